@@ -678,8 +678,14 @@ int tide_b200_set_tma_ctas(int max_ctas);
  * three blocks (64 steps, or the next multiple of the even snapshot
  * interval) as one captured graph replayed per block instead of two launches
  * per step; the step-indexed pointers move with a device-side block counter.
- * Results are bit-identical either way.  1 = on (default), 0 = off.  Returns
- * the previous setting; process-wide, takes effect at the next call. */
+ * Stencil-2 float forward, forward_with_storage (device history or none) and
+ * backward calls of small problems (8192 cells a shot or more, at most 2^19
+ * cells in all, shared coefficients) run as one launch instead; they too need
+ * this switch on.  Fields, receivers, snapshots and source gradients are
+ * bit-identical either way; so are model gradients, except that such a call
+ * with several shots may sum its image terms in another order.  1 = on
+ * (default), 0 = off.  Returns the previous setting; process-wide, takes effect
+ * at the next call. */
 int tide_b200_set_step_graphs(int on);
 
 /* Graph replays issued so far by this process (each one block of steps). */

@@ -1,0 +1,142 @@
+"""Resident time loops (csrc/tm2d_res.cuh) against the per-step kernels.
+
+Calls of 8192 cells or more per shot and at most 2^19 cells in all run every step
+in one cooperative launch; with step graphs off the same call runs one launch per
+half step.  Fields, memories, receivers, snapshots and source gradients must be
+bit-identical for every slab and group shape; model gradients too where one group
+holds all shots (the same step-major sums).  With several groups the sums are
+taken in another order: n = nt x shots terms of either sign, each partial sum
+rounded once, so the two differ by at most about 2 n 2^-24 of the sum of the
+terms' absolute values, and by its square root in practice; with 45 x 5 terms that
+is 1e-6, against which 1e-5 is asserted.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from cases import clone_problem, random_problem
+from oracle_harness import rel_l2
+from tide_b200 import _native as nat
+from tide_b200 import physics as ph
+from tide_b200 import storage as stg
+from tide_b200 import tm2d
+
+pytestmark = pytest.mark.gpu
+NT = 45
+
+# (model ny, nx, CPML width): one row a slab; column blocks cut by both strips; wide and
+# flat (fewer rows than SMs); narrow and tall; no CPML; unequal widths; the largest size.
+SHAPES = [(96, 96, 10), (97, 131, 8), (33, 400, [3, 11, 0, 6]), (400, 33, 5), (100, 100, 0),
+          (3, 2000, 1), (683, 727, 20)]
+
+
+def _problem(shape, shots, k=1):
+    ny, nx, pml = shape
+    pb = random_problem(900 + ny + shots, ny, nx, shots, NT, pml=pml, n_rec=9, k=k)
+    gen = torch.Generator().manual_seed(ny)
+    for t in pb.fields[:3]:
+        t.copy_(1e-3 * torch.randn(t.shape, generator=gen))
+    for t, dim in zip(pb.fields[3:], (1, 0, 0, 1)):
+        t.copy_(1e-3 * torch.randn(t.shape, generator=gen))
+        ph.zero_interior(t, pb.fd_pad, pb.pml_width, dim)
+    # duplicate, unused, edge and boundary-row points
+    si = torch.cat([pb.sources_i, pb.sources_i, torch.full((shots, 1), -1),
+                    torch.full((shots, 1), pb.nx)], 1)
+    pb.sources_i, pb.n_src = si.contiguous(), 4
+    pb.f = torch.randn((NT, shots, 4), generator=gen).reshape(-1).contiguous()
+    ri = pb.receivers_i.clone()
+    ri[0, 1] = ri[0, 0]
+    ri[-1, 2], ri[-1, 3], ri[0, 4] = -1, pb.ny * pb.nx - 1, 0
+    ri[:, 5] = pb.sources_i[:, 0]
+    pb.receivers_i = ri.contiguous()
+    return pb
+
+
+def _fits(pb):
+    return pb.ny * pb.nx >= 8192 and pb.n_shots * pb.ny * pb.nx <= 1 << 19
+
+
+def _launches(resident, call):
+    lib = nat.load()
+    prev = nat.set_step_graphs(resident)
+    n0 = lib.tide_b200_launch_count()
+    try:
+        out = call()
+        torch.cuda.synchronize()
+    finally:
+        nat.set_step_graphs(prev)
+    return out, lib.tide_b200_launch_count() - n0
+
+
+def _forward(pb, dev, fmt, k):
+    g = clone_problem(pb, dev)
+    r = torch.zeros((NT, g.n_shots, g.n_rec), device=dev)
+    if fmt is None:
+        tm2d.native_forward(g, g.ca, g.cb, g.f, r, 0, NT)
+        return [r, *g.fields]
+    g.grad_interval = k
+    sdt = torch.bfloat16 if fmt else torch.float32
+    sn = stg.allocate(stg.STORAGE_DEVICE, sdt, fmt, -(-NT // k), g.n_shots, g.ny, g.nx, dev, True,
+                      True)
+    sn.ey_dev.zero_()
+    sn.curl_dev.zero_()
+    tm2d._run_forward_storage(g, g.ca, g.cb, g.f, r, sn, True, True, None, 0)
+    return [r, *g.fields, sn.ey_dev.clone(), sn.curl_dev.clone()]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shots", [1, 2, 5])
+@pytest.mark.parametrize("fmt,k", [(None, 1), (0, 1), (1, 3)])
+def test_forward_equals_per_step_kernels(cuda_device, shape, shots, fmt, k):
+    pb = _problem(shape, shots, k)
+    if not _fits(pb):
+        pytest.skip("larger than a resident call")
+    a, n_a = _launches(False, lambda: _forward(pb, cuda_device, fmt, k))
+    b, n_b = _launches(True, lambda: _forward(pb, cuda_device, fmt, k))
+    assert n_a >= 2 * NT and n_b <= 2  # the resident path ran
+    for i, (x, y) in enumerate(zip(a, b)):
+        assert torch.equal(x, y), f"output {i}"
+    assert nat.device_status(cuda_device) == 0
+
+
+def _backward(pb, dev, fmt, k, bg, chunk):
+    g = clone_problem(pb, dev)
+    g.grad_interval = k
+    gen = torch.Generator(device=dev).manual_seed(3)
+    sdt = torch.bfloat16 if fmt else torch.float32
+    sn = stg.allocate(stg.STORAGE_DEVICE, sdt, fmt, -(-NT // k), bg or g.n_shots, g.ny, g.nx, dev,
+                      True, True)
+    for t in (sn.ey_dev, sn.curl_dev):
+        t.copy_(torch.randn(t.shape, generator=gen, device=dev))
+    gr = torch.randn((NT, g.n_shots, g.n_rec), generator=gen, device=dev)
+    st = tm2d._AdjointState(g, True, True)
+    for t, f in zip(st.lam, g.fields):
+        t.copy_(f)
+    for t in st.lam[3:]:  # cells no step updates (outermost rows and columns)
+        t[:, 0] = t[:, -1] = 0
+        t[:, :, 0] = t[:, :, -1] = 0
+    for s in range(NT, 0, -chunk):
+        tm2d._backward_call(g, g.ca, g.cb, gr, st, tm2d._snap_ptrs(sn), 0, fmt, sn.shot_bytes, True,
+                            True, s, min(chunk, s), None, bg)
+    return [st.grad_f, *st.lam], [st.grad_ca, st.grad_cb]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shots", [1, 2, 5])
+@pytest.mark.parametrize("fmt,k,bg,chunk", [(0, 1, None, NT), (1, 3, None, 12), (0, 2, 1, NT)])
+def test_adjoint_equals_per_step_kernels(cuda_device, shape, shots, fmt, k, bg, chunk):
+    pb = _problem(shape, shots, k)
+    if not _fits(pb):
+        pytest.skip("larger than a resident call")
+    (a, ga), _ = _launches(False, lambda: _backward(pb, cuda_device, fmt, k, bg, chunk))
+    (b, gb), n_b = _launches(True, lambda: _backward(pb, cuda_device, fmt, k, bg, chunk))
+    assert n_b <= 4 * -(-NT // chunk)
+    for i, (x, y) in enumerate(zip(a, b)):
+        assert torch.equal(x, y), f"output {i}"
+    for x, y in zip(ga, gb):
+        assert rel_l2(y, x) <= 1e-5
+        if shots == 1:
+            assert torch.equal(x, y)
+    assert nat.device_status(cuda_device) == 0

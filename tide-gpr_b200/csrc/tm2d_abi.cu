@@ -25,6 +25,7 @@
 #include "tm2d_fused.cuh"
 #include "tm2d_s2.cuh"
 #include "tm2d_tma.cuh"
+#include "tm2d_res.h"
 #include "tb_store.cuh"
 
 namespace tb {
@@ -780,6 +781,18 @@ inline bool fused_pays(int64_t n_shots, int64_t cells) {
   return t >= 0 && 3 * n_shots * cells * (int64_t)sizeof(float) > t;
 }
 
+// Resident time loops (tm2d_res.cuh): used where the library chooses the path
+// itself, i.e. with step graphs on, the fused forward neither forced (0) nor
+// excluded (negative threshold), and no kernel profile being taken (its samples
+// are of the per-step kernels).
+inline bool res_allowed(cudaStream_t st) {
+  return g_step_graphs.load() && g_fused_min_bytes.load() > 0 && !ProfileScope(st).on();
+}
+inline int *res_err_word() {
+  void *p = nullptr;
+  return TB_CUDA(cudaGetSymbolAddress(&p, g_tide_dev_err)) ? nullptr : static_cast<int *>(p);
+}
+
 template <typename T, int ST>
 void tm_forward(TIDE_TM_FORWARD_ARGS(T)) {
   (void)dt; (void)step_ratio; (void)n_threads;
@@ -827,6 +840,12 @@ void tm_forward(TIDE_TM_FORWARD_ARGS(T)) {
       if (TB_CUDA(cudaGetLastError())) return;
       qr.finish();
       return;
+    }
+    if (db.n_poles == 0 && L.has_domain && res_allowed(st)) {
+      const ResFwdCall rc{L.g, ca, cb, cq, {ey, hx, hz, m_ey_x, m_ey_z, m_hx_z, m_hz_x},
+                          sources_i, receivers_i, n_sources_per_shot, n_receivers_per_shot, f, r,
+                          nullptr, nullptr, false, start_t, nt, 1, st, res_err_word()};
+      if (res_forward(rc) != ResRun::kNotTaken) return;
     }
     if (db.n_poles == 0 && L.has_domain && nt > 0 && fused_pays(n_shots, L.g.N)) {
       // Fused one-launch-per-step path.
@@ -905,6 +924,15 @@ void tm_forward_with_storage(TIDE_TM_FORWARD_WITH_STORAGE_ARGS(T)) {
   if constexpr (is_float<T>() && ST == 2) qpath = L.has_domain && QRun<false>::eligible(L.g, nt);
   const bool fused = !qpath && is_float<T>() && ST == 2 && L.has_domain && nt > 0 &&
                      fused_pays(n_shots, L.g.N);
+  if constexpr (is_float<T>() && ST == 2) {
+    if (!qpath && L.has_domain && !sr.host_side && res_allowed(st)) {
+      const ResFwdCall rc{L.g, ca, cb, cq, {ey, hx, hz, m_ey_x, m_ey_z, m_hx_z, m_hz_x},
+                          sources_i, receivers_i, n_sources_per_shot, n_receivers_per_shot, f, r,
+                          sr.want ? sr.s1[0] : nullptr, sr.want ? sr.s1[1] : nullptr, sr.bf16,
+                          start_t, nt, step_ratio, st, res_err_word()};
+      if (res_forward(rc) != ResRun::kNotTaken) return;
+    }
+  }
   PitchedFwd pf;
   QRun<false> qr;
   if constexpr (is_float<T>()) {
@@ -1063,7 +1091,19 @@ void tm_backward(TIDE_TM_BACKWARD_ARGS(T), int64_t background_n_shots) {
   cudaStream_t st = as_stream(compute_stream);
   // one launch per step on the TMA path (float, stencil 2, unbatched)
   bool qpath = false;
-  if constexpr (is_float<T>() && ST == 2) qpath = L.has_domain && QRun<true>::eligible(L.g, nt);
+  if constexpr (is_float<T>() && ST == 2) {
+    qpath = L.has_domain && QRun<true>::eligible(L.g, nt);
+    if (!qpath && L.has_domain && res_allowed(st) && (!grads || storage_mode == 0)) {
+      const ResAdjCall rc{L.g, ca, cb, cq,
+                          {lambda_ey, lambda_hx, lambda_hz, m_lambda_ey_x, m_lambda_ey_z,
+                           m_lambda_hx_z, m_lambda_hz_x},
+                          sources_i, receivers_i, n_sources_per_shot, n_receivers_per_shot,
+                          grad_r, grad_f, grads && ca_requires_grad ? ey_store_1 : nullptr,
+                          grads && cb_requires_grad ? curl_store_1 : nullptr, bf16, bg_shots,
+                          grad_ca, grad_cb, start_t, nt, step_ratio, st, res_err_word()};
+      if (res_backward(rc) != ResRun::kNotTaken) return;
+    }
+  }
   QRun<true> qr;
   if constexpr (is_float<T>()) {
     float *const fl[3] = {lambda_ey, lambda_hx, lambda_hz};

@@ -806,7 +806,7 @@ __device__ __forceinline__ int point_tile_of(int64_t idx, int s, int nx, const P
   return (s * t.tiles_y + y / t.tile_h) * t.tiles_x + (x + t.xoff) / t.tile_w;
 }
 
-__global__ void k_points_count(const int64_t *__restrict__ idx, int n_per_shot, int n_shots,
+static __global__ void k_points_count(const int64_t *__restrict__ idx, int n_per_shot, int n_shots,
                                int64_t N, int nx, PointTiles pt, int *__restrict__ count) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_per_shot * n_shots) return;
@@ -821,7 +821,7 @@ __global__ void k_points_count(const int64_t *__restrict__ idx, int n_per_shot, 
 
 // Per tile row i = shot * tiles_y + tile row: does any tile of the row hold a
 // point of either list?  (start arrays are exclusive scans over the tiles.)
-__global__ void k_points_rowflags(const int *__restrict__ s_start, const int *__restrict__ r_start,
+static __global__ void k_points_rowflags(const int *__restrict__ s_start, const int *__restrict__ r_start,
                                   int tiles_x, int n_rows, unsigned char *__restrict__ flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows) return;
@@ -833,7 +833,7 @@ __global__ void k_points_rowflags(const int *__restrict__ s_start, const int *__
 }
 
 // Exclusive scan of count[0..n) into start[0..n] by one block of 1024 threads.
-__global__ void __launch_bounds__(1024) k_points_scan(const int *__restrict__ count,
+static __global__ void __launch_bounds__(1024) k_points_scan(const int *__restrict__ count,
                                                      int *__restrict__ start, int n) {
   __shared__ int part[1024];
   const int t = threadIdx.x;
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(1024) k_points_scan(const int *__restrict__ co
 
 // Place each entry at start[tile] + (its rank among earlier entries of the
 // same shot and tile), so every tile lists its entries in ascending order.
-__global__ void k_points_fill(const int64_t *__restrict__ idx, int n_per_shot, int n_shots,
+static __global__ void k_points_fill(const int64_t *__restrict__ idx, int n_per_shot, int n_shots,
                               int64_t N, int nx, PointTiles pt, const int *__restrict__ start,
                               int *__restrict__ cell,
                               int *__restrict__ ent) {

@@ -1,0 +1,300 @@
+// Host side of the resident TM2D time loops (tm2d_res.cuh): which calls run
+// resident, how their grid is cut into slabs, and the launch.
+#include "tm2d_res.h"
+
+#include <algorithm>
+
+#include "tb_common.cuh"
+#include "tm2d_res.cuh"
+
+namespace tb {
+namespace {
+
+struct Device {
+  int dev = 0, sms = 0, smem = 0;
+  bool coop = false;
+};
+
+bool device_of(Device &d) {
+  int coop = 0;
+  if (TB_CUDA(cudaGetDevice(&d.dev)) ||
+      TB_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, d.dev)) ||
+      TB_CUDA(cudaDeviceGetAttribute(&d.smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, d.dev)) ||
+      TB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d.dev)))
+    return false;
+  d.coop = coop != 0;
+  d.smem -= 2048;  // the kernels' static shared memory
+  return true;
+}
+
+// Cuts ny rows into at most P slabs of near-equal cost (an interior row costs 1,
+// a y-strip row `strip`), each within the shared memory limit; returns the
+// largest slab cost, or -1.  smem(ya, yb): bytes of a slab.
+template <typename Smem>
+double cut_rows(ResPlan &pl, const TMGeom<float> &g, int P, double strip, size_t limit, Smem smem) {
+  auto row_cost = [&](int y) { return y < g.pml_y0 || y >= g.pml_y1h ? strip : 1.0; };
+  double total = 0;
+  for (int y = 0; y < g.ny; ++y) total += row_cost(y);
+  auto greedy = [&](double cap, int *row) -> int {
+    int n = 0, y = 0;
+    while (y < g.ny) {
+      if (n == P) return -1;
+      if (row) row[n] = y;
+      const int y0 = y;
+      double c = 0;
+      while (y < g.ny && y - y0 < kResMaxRows) {
+        const double rc = row_cost(y);
+        if (y > y0 && c + rc > cap + 1e-9) break;
+        if (smem(y0, y + 1) > limit) {
+          if (y == y0) return -1;
+          break;
+        }
+        c += rc;
+        ++y;
+      }
+      ++n;
+    }
+    if (row) row[n] = g.ny;
+    return n;
+  };
+  double lo = total / P, hi = total;
+  if (greedy(hi, nullptr) < 0) return -1;
+  for (int i = 0; i < 30; ++i) {
+    const double mid = 0.5 * (lo + hi);
+    if (greedy(mid, nullptr) < 0) lo = mid;
+    else hi = mid;
+  }
+  pl.P = greedy(hi, pl.row);
+  if (pl.P < 1) return -1;
+  double worst = 0;
+  for (int p = 0; p < pl.P; ++p) {
+    double c = 0;
+    for (int y = pl.row[p]; y < pl.row[p + 1]; ++y) c += row_cost(y);
+    worst = std::max(worst, c);
+  }
+  return worst;
+}
+
+// Microseconds of one step of one round (a group on every sub-grid), by which
+// shapes are compared: a fixed part (halo exchange, barriers, the latency of one
+// task) and a part per 32-column block, row and shot of the largest slab, smaller
+// with more shots per task (the loads and chains of a task's shots overlap).
+// Fitted at 1965 MHz: 117 x 117, 1 shot 2.2; 161 x 201, 2 shots as one group 3.7,
+// as two 3.5; 342 x 528, 6 shots G = 3 10.5, G = 2 13.1, G = 1 17.2.
+constexpr double kStepUs = 2.2, kUnitUs[4] = {0.047, 0.031, 0.025, 0.026};
+constexpr double kStripRow = 3.0;  // cost of a y-strip row in interior rows
+
+// Chooses shots per group, sub-grids and slabs; false: no shape fits.
+bool plan_res(ResPlan &best, const TMGeom<float> &g, const Device &d, bool adj) {
+  const int XB = (g.nx + 31) / 32, XW = g.pml_x0 + g.nx - g.pml_x1h;
+  const int S = g.n_shots;
+  double best_t = 1e300;
+  for (int G = 1; G <= std::min(4, S); ++G) {
+    const int ngroups = (S + G - 1) / G;
+    if (G > 1 && (S + ngroups - 1) / ngroups < G) continue;  // same groups as a smaller G
+    const int K = 3 * G + (adj ? 5 : 3);
+    auto smem = [&](int ya, int yb) {
+      const int end = adj ? res_adj_smem(yb - ya, XB, XW, G, K, res_adj_ystrip(g, ya, yb)).end
+                          : res_smem(yb - ya, XB, XW, G, K, res_ystrip(g, ya, yb)).end;
+      return (size_t)end * sizeof(float);
+    };
+    for (int Q = 1; Q <= std::min(ngroups, d.sms); ++Q) {
+      ResPlan pl;
+      const int P = std::min({d.sms / Q, kResMaxCta, g.ny});
+      if (P < 1) break;
+      const int rounds = (ngroups + Q - 1) / Q;
+      const double unit = kUnitUs[G - 1] * XB * G;
+      if (rounds * (kStepUs + unit * g.ny / P) >= best_t) continue;  // before the strips
+      const double rows = cut_rows(pl, g, P, kStripRow, (size_t)d.smem, smem);
+      if (rows < 0) continue;
+      const double t = rounds * (kStepUs + unit * rows);
+      if (t >= best_t) continue;
+      best_t = t;
+      pl.Q = Q;
+      pl.G = G;
+      pl.n_groups = ngroups;
+      pl.XB = XB;
+      pl.XW = XW;
+      for (int p = 0; p < pl.P; ++p) pl.smem = std::max(pl.smem, smem(pl.row[p], pl.row[p + 1]));
+      best = pl;
+    }
+  }
+  if (best_t >= 1e300) return false;
+  int R = 0;
+  for (int p = 0; p < best.P; ++p) R = std::max(R, best.row[p + 1] - best.row[p]);
+  // A warp per task (a straight-line task has up to UR rows), as many as give
+  // every warp the same number of tasks, whole quarters of the SM (553 x 1065, 8
+  // shots: 16 warps 49.9 us a step, 17 warps 56.1).
+  const int most = (adj ? kResAdjThreads : kResFwdThreads) / 32, ur = best.G == 1 ? 4 : 2;
+  const int tasks = XB * ((R + ur - 1) / ur);
+  const int rounds = (tasks + most - 1) / most;
+  best.warps = std::max(4, std::min(most, (tasks + rounds - 1) / rounds));
+  if (best.warps > 8) best.warps = best.warps / 4 * 4;
+  return true;
+}
+
+struct Scratch {
+  void *p = nullptr;
+  cudaStream_t st = nullptr;
+  ~Scratch() {
+    if (p) cudaFreeAsync(p, st);
+  }
+};
+
+template <typename Args>
+ResRun launch(void (*k)(const Args), const Args &a, cudaStream_t st) {
+  if (TB_CUDA(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)a.pl.smem)))
+    return ResRun::kFailed;
+  void *args[] = {const_cast<Args *>(&a)};
+  const cudaError_t e = cudaLaunchCooperativeKernel(
+      (const void *)k, dim3((unsigned)(a.pl.P * a.pl.Q)), dim3((unsigned)(32 * a.pl.warps)), args,
+      a.pl.smem, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device reports
+    cudaGetLastError();
+    return ResRun::kNotTaken;
+  }
+  if (TB_CUDA(e)) return ResRun::kFailed;
+  count_launches(1);
+  return ResRun::kDone;
+}
+
+template <typename Sn>
+ResRun run_forward(const ResFwdCall &c, const ResPlan &pl) {
+  const TMGeom<float> &g = c.g;
+  const int64_t ns = c.src_i && c.n_src > 0 ? c.n_src : 0, nr = c.rec_i && c.n_rec > 0 ? c.n_rec : 0;
+  const size_t ll = (size_t)2 * pl.Q * std::max(0, pl.P - 1) * 2 * pl.G * g.nx * 8;
+  const size_t lists = (size_t)pl.P * pl.Q * pl.G * (size_t)(3 * ns + 2 * nr) * 4;
+  if (lists > ((size_t)256 << 20)) return ResRun::kNotTaken;
+  Scratch sc;
+  sc.st = c.st;
+  if (TB_CUDA(pool_malloc(&sc.p, ll + lists + 16, c.st))) return ResRun::kFailed;
+  if (ll && TB_CUDA(cudaMemsetAsync(sc.p, 0, ll, c.st))) return ResRun::kFailed;
+  ResFwdArgs<Sn> a{};
+  a.g = g;
+  a.pl = pl;
+  a.ca = c.ca; a.cb = c.cb; a.cq = c.cq;
+  a.ey = c.fields[0]; a.hx = c.fields[1]; a.hz = c.fields[2]; a.mex = c.fields[3];
+  a.mez = c.fields[4]; a.mhx = c.fields[5]; a.mhz = c.fields[6];
+  a.src = ResPoints{c.src_i, (int)ns};
+  a.rec = ResPoints{c.rec_i, (int)nr};
+  a.f = c.f;
+  a.r = c.r;
+  a.est = static_cast<Sn *>(c.est);
+  a.cst = static_cast<Sn *>(c.cst);
+  a.t0 = c.t0;
+  a.nt = (int)c.nt;
+  a.ratio = (int)c.ratio;
+  a.ll = static_cast<unsigned long long *>(sc.p);
+  a.lists = reinterpret_cast<int *>(static_cast<char *>(sc.p) + ll);
+  a.err = c.err;
+  switch (pl.G) {
+    case 1: return launch(k_res_fwd<Sn, 1>, a, c.st);
+    case 2: return launch(k_res_fwd<Sn, 2>, a, c.st);
+    case 3: return launch(k_res_fwd<Sn, 3>, a, c.st);
+    default: return launch(k_res_fwd<Sn, 4>, a, c.st);
+  }
+}
+
+template <typename Sn>
+ResRun run_backward(const ResAdjCall &c, const ResPlan &pl) {
+  const TMGeom<float> &g = c.g;
+  const int64_t ns = c.src_i && c.n_src > 0 ? c.n_src : 0, nr = c.rec_i && c.n_rec > 0 ? c.n_rec : 0;
+  const bool many = pl.n_groups > 1;
+  const size_t ll = (size_t)2 * pl.Q * std::max(0, pl.P - 1) * 2 * pl.G * g.nx * 8;
+  const size_t lists = (size_t)pl.P * pl.Q * pl.G * (size_t)(2 * ns + 3 * nr) * 4;
+  const size_t acc = many ? (size_t)pl.Q * (size_t)g.N * 4 : 0;
+  const int n_acc = (c.est ? 1 : 0) + (c.cst ? 1 : 0);
+  if (lists > ((size_t)256 << 20)) return ResRun::kNotTaken;
+  Scratch sc;
+  sc.st = c.st;
+  if (TB_CUDA(pool_malloc(&sc.p, ll + n_acc * acc + lists + 16, c.st))) return ResRun::kFailed;
+  if (ll && TB_CUDA(cudaMemsetAsync(sc.p, 0, ll, c.st))) return ResRun::kFailed;
+  char *m = static_cast<char *>(sc.p) + ll;
+  ResAdjArgs<Sn> a{};
+  a.g = g;
+  a.pl = pl;
+  a.ca = c.ca; a.cb = c.cb; a.cq = c.cq;
+  a.ey = c.fields[0]; a.hx = c.fields[1]; a.hz = c.fields[2]; a.mex = c.fields[3];
+  a.mez = c.fields[4]; a.mhx = c.fields[5]; a.mhz = c.fields[6];
+  a.src = ResPoints{c.src_i, (int)ns};
+  a.rec = ResPoints{c.rec_i, (int)nr};
+  a.gr = c.grad_r;
+  a.gf = c.grad_f;
+  a.est = static_cast<const Sn *>(c.est);
+  a.cst = static_cast<const Sn *>(c.cst);
+  a.bg = c.bg;
+  a.gca = c.est ? c.grad_ca : nullptr;
+  a.gcb = c.cst ? c.grad_cb : nullptr;
+  if (many && c.est) {
+    a.gca = reinterpret_cast<float *>(m);
+    m += acc;
+  }
+  if (many && c.cst) {
+    a.gcb = reinterpret_cast<float *>(m);
+    m += acc;
+  }
+  a.kscale = (float)c.ratio;
+  a.t1 = c.t1;
+  a.nt = (int)c.nt;
+  a.ratio = (int)c.ratio;
+  a.ll = static_cast<unsigned long long *>(sc.p);
+  a.lists = reinterpret_cast<int *>(m);
+  a.err = c.err;
+  const ResRun r = pl.G == 1   ? launch(k_res_adj<Sn, 1>, a, c.st)
+                   : pl.G == 2 ? launch(k_res_adj<Sn, 2>, a, c.st)
+                   : pl.G == 3 ? launch(k_res_adj<Sn, 3>, a, c.st)
+                               : launch(k_res_adj<Sn, 4>, a, c.st);
+  if (r != ResRun::kDone || !many) return r;
+  const unsigned blocks = (unsigned)std::min<int64_t>((g.N + 255) / 256, 1184);
+  if (c.est) k_res_combine<<<blocks, 256, 0, c.st>>>(c.grad_ca, a.gca, pl.Q, g.N);
+  if (c.cst) k_res_combine<<<blocks, 256, 0, c.st>>>(c.grad_cb, a.gcb, pl.Q, g.N);
+  count_launches(n_acc);
+  return TB_CUDA(cudaGetLastError()) ? ResRun::kFailed : r;
+}
+
+// Largest resident call, shots x cells.  161 x 201, 2 shots (65 k): 4.6 us a step
+// forward and 7.5 adjoint against 6.9 and 11.6 for the per-step kernels; 342 x 528,
+// 6 shots (1.08 M): 14.2 against 15.3 forward; 430 x 742, 5 shots (1.6 M): 28.5
+// against 34 adjoint on zero fields; 553 x 1065, 4 shots (2.4 M): 55 against 39
+// adjoint.  Grids below kResMinCells keep the step blocks' graph replay.
+constexpr int64_t kResMaxShotCells = (int64_t)1 << 19;
+
+// Common conditions of a resident call.
+bool res_eligible(const TMGeom<float> &g, int64_t nt, int64_t n_src, int64_t n_rec,
+                  cudaStream_t st) {
+  if (g.ca_b || g.cb_b || g.cq_b || g.nx < 2 || g.ny < 2) return false;
+  if (g.N < kResMinCells || g.n_shots * g.N > kResMaxShotCells) return false;
+  // (an upper bound on nt keeps one launch under a second)
+  if (nt < 8 || nt > (1 << 16) || (int64_t)g.n_shots * nt > ((int64_t)1 << 30)) return false;
+  if (std::max(n_src, n_rec) * g.n_shots > (1 << 30)) return false;
+  if (g.pml_y0 < 0 || g.pml_x0 < 0 || g.pml_x1h > g.nx || g.pml_x0 > g.pml_x1h) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
+}  // namespace
+
+ResRun res_forward(const ResFwdCall &c) {
+  if (!res_eligible(c.g, c.nt, c.n_src, c.n_rec, c.st)) return ResRun::kNotTaken;
+  Device d;
+  if (!device_of(d)) return ResRun::kFailed;
+  ResPlan pl;
+  if (!d.coop || !plan_res(pl, c.g, d, false)) return ResRun::kNotTaken;
+  return c.bf16 ? run_forward<__nv_bfloat16>(c, pl) : run_forward<float>(c, pl);
+}
+
+ResRun res_backward(const ResAdjCall &c) {
+  if (!res_eligible(c.g, c.nt, c.n_src, c.n_rec, c.st)) return ResRun::kNotTaken;
+  Device d;
+  if (!device_of(d)) return ResRun::kFailed;
+  ResPlan pl;
+  if (!d.coop || !plan_res(pl, c.g, d, true)) return ResRun::kNotTaken;
+  return c.bf16 ? run_backward<__nv_bfloat16>(c, pl) : run_backward<float>(c, pl);
+}
+
+}  // namespace tb

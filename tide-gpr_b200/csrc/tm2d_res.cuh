@@ -1,0 +1,1532 @@
+// Resident TM2D time loops (stencil 2, FP32, unbatched model): one cooperative
+// launch runs every time step of a call with the state held in shared memory.
+//
+// The grid of a shot is cut into slabs of whole rows, one CTA (one SM) per
+// slab; a CTA holds its slab's Ey, Hx, Hz of G shots, the CPML memories of its
+// strips and the model coefficients in shared memory for the whole call, so a time
+// step touches device memory for snapshots, sources and receivers only.  A step needs one exchange between neighbouring slabs: the
+// boundary rows of Ey.  A CTA keeps its own copy of the H-x row (and of that
+// row's CPML memory) just above its slab and advances it with the same
+// operations as its owner, so H-x never crosses.
+//
+// Exchange.  Each boundary value travels as one 64-bit word {step tag, value}
+// through L2 (two slots by step parity); the thread that owns the column on
+// the other side polls that word, so no flag, fence or grid-wide barrier is
+// needed.  A slot is rewritten two steps later, which its writer reaches only
+// after it has read a value the reader published past its last read of the
+// slot.  All CTAs are co-resident (cooperative launch); every poll is bounded,
+// after which the CTA sets the device error word and stops waiting.
+//
+// What bounds it.  A step of the per-step kernels on a small grid is two launches
+// of 2 to 7 us each, most of it launch and first-load latency.  Here a step is one
+// exchange through L2 (about 0.6 us), two block barriers and the latency of the
+// slowest task, a strip row: 117 x 117, 1 shot 2.2 us a step against 5.9; 161 x
+// 201, 2 shots 4.6 forward and 7.5 adjoint against 6.9 and 11.6.  On large grids
+// the tasks' address and predicate arithmetic (147 warp instructions per 32 cells)
+// makes it lose to the per-step kernels, which fill the SMs (see kResMaxShotCells).
+//
+// Shared-memory layout.  Columns in blocks of 32 (one warp row); a block holds
+// the K arrays of its 32 columns side by side ([row][block][array][32]), so
+// all arrays of a cell are at compile-time offsets from one address and every
+// access is conflict-free.
+//
+// Values are computed with the operations of the per-step kernels
+// (tm2d_s2.cuh) in the same order: results are bit-identical to them.
+#pragma once
+
+#include <type_traits>
+
+#include "tm2d_kernels.cuh"
+
+namespace tb {
+
+constexpr int kResMaxCta = 160;     // slabs of one launch (B200: 148 SMs)
+constexpr int kResFwdThreads = 640;  // most threads of a forward CTA (96 registers each)
+constexpr int kResAdjThreads = 512;  // ... of an adjoint CTA (128)
+constexpr int kResSpin = 1 << 22;   // polls of one halo word before giving up (seconds)
+constexpr int64_t kResMinCells = 8192;  // cells of a shot's grid from which calls run resident
+constexpr int kResMaxRows = 1024;   // rows of a slab (adjoint row flags)
+
+// Shape of one resident launch.  CTA blockIdx.x works on slab p = blockIdx.x %
+// P of sub-grid q = blockIdx.x / P; sub-grid q runs shot groups q, q + Q, ...
+struct ResPlan {
+  int P = 0, Q = 0, G = 0, n_groups = 0;
+  int XB = 0;       // 32-column blocks of a row
+  int XW = 0;       // columns of both x strips (compact x memories)
+  int warps = 0;
+  size_t smem = 0;
+  int row[kResMaxCta + 1] = {};  // slab p owns rows [row[p], row[p + 1])
+};
+
+// First shot of group j of n (sizes differ by at most one).
+__host__ __device__ inline int res_group_begin(int j, int n, int S) {
+  return (int)((int64_t)j * S / n);
+}
+
+// Point entries of one kind (sources or receivers).
+template <int N> using IntC = std::integral_constant<int, N>;
+
+struct ResPoints {
+  const int64_t *idx;  // [S, n] flat cells (negative: unused)
+  int n;
+};
+
+template <typename Sn> struct ResFwdArgs {
+  TMGeom<float> g;
+  ResPlan pl;
+  const float *ca, *cb, *cq;
+  float *ey, *hx, *hz, *mex, *mez, *mhx, *mhz;
+  ResPoints src, rec;
+  const float *f;  // [steps, S, n_src] of step 0 of the call's time axis
+  float *r;
+  Sn *est, *cst;   // device histories (slot q at q * S * N), null: not stored
+  int64_t t0;
+  int nt, ratio;   // ratio: steps between stored steps
+  unsigned long long *ll;
+  int *lists;      // per CTA: (cell, entry, next) of sources, then (cell, entry) of receivers
+  int *err;
+};
+
+__device__ __forceinline__ unsigned long long ll_load(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ll_store(unsigned long long *p, float v, unsigned tag) {
+  const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+// Value of a halo word once it carries `tag`; `v` is its first read.  Bounded:
+// after kResSpin polls (or once the CTA has given up) it returns what is there.
+__device__ __forceinline__ float ll_wait(const unsigned long long *p, unsigned tag,
+                                         unsigned long long v, volatile int *dead, int *err) {
+  if ((unsigned)(v >> 32) != tag) {
+    int n = 0;
+    do {
+      if (*dead || ++n > kResSpin) {
+        if (!*dead) {
+          *dead = 1;
+          atomicOr(err, 2);
+        }
+        break;
+      }
+      v = ll_load(p);
+    } while ((unsigned)(v >> 32) != tag);
+  }
+  return __uint_as_float((unsigned)v);
+}
+
+// d / k for a CPML kappa, correctly rounded.  inv is k's rounded reciprocal (0:
+// k outside [1/8, 8], plain division).  Markstein's method (P. Markstein, IBM J.
+// Res. Dev. 34, 1990): a quotient estimate is corrected twice by its residual,
+// which a fused multiply-add gives exactly away from underflow.  Numerators down
+// to 2^-123 are scaled by 2^60 for that (the quotient is still normal); smaller
+// ones, zeros aside, and huge ones take the plain division.  The compiler's
+// division leaves its short path for numerators far below 1, which is what the
+// strips hold until the wave arrives: the strip rows then set a step's time.
+__device__ __forceinline__ float res_div(float d, float k, float inv) {
+  const float ad = fabsf(d);
+  const bool small = ad < 0x1p-100f;
+  const float n = small ? d * 0x1p60f : d;
+  float q = n * inv;
+  q = __fmaf_rn(__fmaf_rn(-k, q, n), inv, q);
+  q = __fmaf_rn(__fmaf_rn(-k, q, n), inv, q);
+  q = small ? q * 0x1p-60f : q;
+  const bool plain = !(ad >= 0x1p-123f && ad <= 0x1p100f && inv != 0.f);
+  if (plain && d != 0.f) q = d / k;
+  return d == 0.f ? d : q;
+}
+__device__ __forceinline__ float res_inv(float k) {
+  return k >= 0.125f && k <= 8.f ? 1.f / k : 0.f;
+}
+// CPML profile values of one row or column: b, a, kappa and its reciprocal.
+struct ResProf {
+  float b, a, k, i;
+};
+// Tables of a CTA: half-point and integer profiles of its rows -1 .. R and of the
+// strip columns (compact index).
+__device__ __forceinline__ void res_profiles(const TMGeom<float> &g, ResProf *yh, ResProf *ye,
+                                             ResProf *xh, ResProf *xe, int ya, int R, int XW) {
+  for (int i = threadIdx.x; i < R + 2; i += blockDim.x) {
+    const int y = ya - 1 + i;
+    if (y < 0 || y >= g.ny) continue;
+    yh[i] = ResProf{g.byh[y], g.ayh[y], g.kyh[y], res_inv(g.kyh[y])};
+    ye[i] = ResProf{g.by[y], g.ay[y], g.ky[y], res_inv(g.ky[y])};
+  }
+  for (int c = threadIdx.x; c < XW; c += blockDim.x) {
+    const int x = c < g.pml_x0 ? c : c - g.pml_x0 + g.pml_x1h;
+    xh[c] = ResProf{g.bxh[x], g.axh[x], g.kxh[x], res_inv(g.kxh[x])};
+    xe[c] = ResProf{g.bx[x], g.ax[x], g.kx[x], res_inv(g.kx[x])};
+  }
+}
+
+// Ordered list of the entries of shots [s0, s0 + ng) that lie in rows [ya, yb):
+// local cell r * W + x and entry e = s * n + k.  Every thread of the block calls
+// it; returns the count.
+__device__ __forceinline__ int res_list(const ResPoints &pt, int s0, int ng, int ya, int yb, int W,
+                                        int64_t N, int *cell, int *ent, int cap, int *wsum,
+                                        int *err, bool report) {
+  const int tot = pt.n * ng, nthr = blockDim.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t lo = (int64_t)ya * W, hi = (int64_t)yb * W;
+  int n = 0;
+  for (int b = 0; b < tot; b += nthr) {
+    const int k = b + threadIdx.x;
+    int64_t v = -1;
+    if (k < tot) v = pt.idx[(int64_t)s0 * pt.n + k];
+    if (v >= N && report) atomicOr(err, 1);
+    const bool in = v >= lo && v < hi;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) wsum[w] = __popc(m);
+    __syncthreads();
+    int off = n, all = 0;
+    for (int i = 0; i < (nthr >> 5); ++i) {
+      if (i < w) off += wsum[i];
+      all += wsum[i];
+    }
+    if (in) {
+      const int pos = off + __popc(m & ((1u << lane) - 1));
+      if (pos < cap) {
+        cell[pos] = (int)(v - lo);
+        ent[pos] = s0 * pt.n + k;
+      }
+    }
+    n += all;
+    __syncthreads();
+  }
+  return min(n, cap);
+}
+
+// f(IntC<n>) for n in 1 .. MAX rows of a straight-line task.
+template <int MAX, typename F> __device__ __forceinline__ void res_rows(int n, F &&f) {
+  if constexpr (MAX > 1) {
+    if (n < MAX) {
+      res_rows<MAX - 1>(n, f);
+      return;
+    }
+  }
+  f(IntC<MAX>());
+}
+
+// Chains the entries of a list that share a cell of one shot, in entry order.
+// next[i]: the following entry of the chain or -1; -2 - (that + 1) when i is not
+// its chain's first entry.
+__device__ __forceinline__ void res_chain(const int *cell, const int *ent, int *next, int n,
+                                          int per_shot) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int c = cell[i], sh = ent[i] / per_shot;
+    bool first = true;
+    for (int j = 0; j < i && first; ++j) first = !(cell[j] == c && ent[j] / per_shot == sh);
+    int nx = -1;
+    for (int j = i + 1; j < n && nx < 0; ++j)
+      if (cell[j] == c && ent[j] / per_shot == sh) nx = j;
+    next[i] = first ? nx : -2 - (nx + 1);
+  }
+}
+__device__ __forceinline__ int res_next(const int *next, int i) {
+  const int v = next[i];
+  return v >= -1 ? v : -3 - v;
+}
+
+// Shared-memory offsets (floats) of one CTA.
+struct ResSmem {
+  int pyh, pye, pxh, pxe;  // profile tables
+  int blk, halo, mzh, mze, mxh, mxe, end;
+};
+// K arrays per block; halo row: H-x of G shots and cq.
+__host__ __device__ inline ResSmem res_smem(int R, int XB, int XW, int G, int K, bool ystrip) {
+  ResSmem s;
+  s.pyh = 0;
+  s.pye = s.pyh + 4 * (R + 2);
+  s.pxh = s.pye + 4 * (R + 2);
+  s.pxe = s.pxh + 4 * XW;
+  s.blk = s.pxe + 4 * XW;
+  s.halo = s.blk + R * XB * K * 32;
+  s.mzh = s.halo + XB * (G + 1) * 32;
+  const int ny = ystrip ? XB * G * 32 : 0;
+  s.mze = s.mzh + (R + 1) * ny;   // m_ey_z: rows -1 .. R - 1
+  s.mxh = s.mze + R * ny;         // m_hx_z: rows 0 .. R - 1
+  s.mxe = s.mxh + G * R * XW;
+  s.end = s.mxe + G * R * XW;
+  return s;
+}
+// Does a slab of the forward (or the row above it) hold y-strip rows?
+__host__ __device__ inline bool res_ystrip(const TMGeom<float> &g, int ya, int yb) {
+  return ya - 1 < g.pml_y0 || yb > g.pml_y1h;
+}
+
+template <typename Sn, int G>
+__global__ void __launch_bounds__(kResFwdThreads, 1)
+k_res_fwd(const __grid_constant__ ResFwdArgs<Sn> a) {
+  constexpr int K = 3 * G + 3;
+  constexpr int UR = G == 1 ? 4 : 2;  // rows in flight of the straight-line path
+  constexpr int EY = 0, HX = G * 32, HZ = 2 * G * 32, CQ = 3 * G * 32, CA = CQ + 32, CB = CQ + 64;
+  extern __shared__ __align__(16) float sm[];
+  __shared__ int s_dead;
+  __shared__ int s_wsum[kResFwdThreads / 32];
+  const TMGeom<float> &g = a.g;
+  const int W = g.nx, ny = g.ny, S = g.n_shots;
+  const int P = a.pl.P, p = blockIdx.x % P, q = blockIdx.x / P;
+  const int ya = a.pl.row[p], yb = a.pl.row[p + 1], R = yb - ya;
+  const int XB = a.pl.XB, XW = a.pl.XW;
+  const bool ystrip = res_ystrip(g, ya, yb);
+  const ResSmem L = res_smem(R, XB, XW, G, K, ystrip);
+  float *const blk = sm + L.blk, *const halo = sm + L.halo;
+  float *const mzh = sm + L.mzh, *const mze = sm + L.mze;
+  float *const mxh = sm + L.mxh, *const mxe = sm + L.mxe;
+  ResProf *const pyh = reinterpret_cast<ResProf *>(sm + L.pyh) + 1;  // [-1]: the row above
+  ResProf *const pye = reinterpret_cast<ResProf *>(sm + L.pye) + 1;
+  ResProf *const pxh = reinterpret_cast<ResProf *>(sm + L.pxh);
+  ResProf *const pxe = reinterpret_cast<ResProf *>(sm + L.pxe);
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int rowst = XB * K * 32;  // floats from one row to the next in blk
+  const bool has_up = p > 0, has_dn = p + 1 < P;
+  // Column blocks [xb_lo, xb_hi) hold no strip cell or grid edge (none when the
+  // slab's rows do): straight-line path, tasks of UR rows.  The others ("general")
+  // run one row a task.  A warp takes tasks warp, warp + nwarps, ...: the n_gen
+  // general ones come first.
+  const bool plain = !ystrip && ya >= 2 && yb < ny;
+  const int xb_lo = plain ? min(XB, (max(g.pml_x0, 1) + 31) / 32) : XB;
+  const int xb_hi = plain ? max(xb_lo, min(g.pml_x1h, W - 1) / 32) : XB;
+  const int n_pl = xb_hi - xb_lo, n_gb = XB - n_pl, n_gen = n_gb * R;
+  const int nwarps = nthr >> 5;
+  const int gen_r0 = n_gb ? warp / n_gb : 0, gen_b0 = n_gb ? warp - gen_r0 * n_gb : 0;
+  const int gen_dr = n_gb ? nwarps / n_gb : 0, gen_db = n_gb ? nwarps - gen_dr * n_gb : 0;
+  // first plain task of this warp and the step to the next, as (block, chunk)
+  const int pl_t0 = warp >= n_gen ? warp - n_gen
+                                  : (nwarps - (n_gen - warp) % nwarps) % nwarps;
+  const int n_ch = (R + UR - 1) / UR;
+  const int pl_c0 = n_pl ? pl_t0 / n_pl : n_ch, pl_b0 = n_pl ? pl_t0 - pl_c0 * n_pl : 0;
+  const int pl_dc = n_pl ? nwarps / n_pl : 0, pl_db = n_pl ? nwarps - pl_dc * n_pl : 0;
+  // halo words: [parity][sub-grid][boundary][direction][shot][W]; boundary b
+  // lies between slabs b and b + 1, direction 0 upwards (first row of b + 1)
+  const int64_t ll_par = (int64_t)a.pl.Q * (P - 1) * 2 * G * W;
+  unsigned long long *const ll_q = a.ll + (int64_t)q * (P - 1) * 2 * G * W;
+  auto ll_at = [&](unsigned tag, int b, int dir) {
+    return ll_q + (tag & 1) * ll_par + ((int64_t)b * 2 + dir) * G * W;
+  };
+  const int n_src = a.src.n, n_rec = a.rec.n;
+  int *const ls = a.lists + (int64_t)blockIdx.x * G * (3 * n_src + 2 * n_rec);
+  int *const s_cell = ls, *const s_ent = s_cell + G * n_src, *const s_next = s_ent + G * n_src;
+  int *const r_cell = s_next + G * n_src, *const r_ent = r_cell + G * n_rec;
+  if (tid == 0) s_dead = 0;
+  res_profiles(g, pyh - 1, pye - 1, pxh, pxe, ya, R, XW);
+
+  for (int i = tid; i < R * XB * 32; i += nthr) {
+    const int x = i % (XB * 32), r = i / (XB * 32);
+    float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+    const int64_t j = (int64_t)(ya + r) * W + x;
+    const bool in = x < W;
+    b[CQ] = in ? __ldg(a.cq + j) : 0.f;
+    b[CA] = in ? __ldg(a.ca + j) : 0.f;
+    b[CB] = in ? __ldg(a.cb + j) : 0.f;
+  }
+  for (int x = tid; x < XB * 32; x += nthr)
+    halo[(x >> 5) * ((G + 1) * 32) + G * 32 + (x & 31)] =
+        (has_up && x < W) ? __ldg(a.cq + (int64_t)(ya - 1) * W + x) : 0.f;
+
+  unsigned tag = 1;  // tag of the halo values the coming step reads
+  for (int grp = q; grp < a.pl.n_groups; grp += a.pl.Q) {
+    const int s0 = res_group_begin(grp, a.pl.n_groups, S);
+    const int ng = res_group_begin(grp + 1, a.pl.n_groups, S) - s0;
+    // ---- state of the group
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      const int64_t sb = (int64_t)(s0 + k) * g.N;
+      const bool on = k < ng;
+      for (int i = tid; i < R * XB * 32; i += nthr) {
+        const int x = i % (XB * 32), r = i / (XB * 32);
+        float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        const bool in = on && x < W;
+        b[EY + k * 32] = in ? a.ey[j] : 0.f;
+        b[HX + k * 32] = in ? a.hx[j] : 0.f;
+        b[HZ + k * 32] = in ? a.hz[j] : 0.f;
+        if (ystrip) {
+          const int o = ((r + 1) * XB + (x >> 5)) * (G * 32) + k * 32 + (x & 31);
+          mzh[o] = in ? a.mez[j] : 0.f;
+          mze[o - XB * G * 32] = in ? a.mhx[j] : 0.f;
+        }
+      }
+      for (int x = tid; x < XB * 32; x += nthr) {
+        const bool in = on && has_up && x < W;
+        const int64_t j = sb + (int64_t)(ya - 1) * W + x;
+        halo[(x >> 5) * ((G + 1) * 32) + k * 32 + (x & 31)] = in ? a.hx[j] : 0.f;
+        if (ystrip) mzh[(x >> 5) * (G * 32) + k * 32 + (x & 31)] = in ? a.mez[j] : 0.f;
+      }
+      for (int i = tid; i < R * XW; i += nthr) {
+        const int c = i % XW, r = i / XW;
+        const int x = c < g.pml_x0 ? c : c - g.pml_x0 + g.pml_x1h;
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        mxh[(k * R + r) * XW + c] = on ? a.mex[j] : 0.f;
+        mxe[(k * R + r) * XW + c] = on ? a.mhz[j] : 0.f;
+      }
+    }
+    // ---- point lists of the group
+    const int ns = n_src > 0 ? res_list(a.src, s0, ng, ya, yb, W, g.N, s_cell, s_ent, G * n_src,
+                                        s_wsum, a.err, p == 0)
+                             : 0;
+    const int nr = n_rec > 0 ? res_list(a.rec, s0, ng, ya, yb, W, g.N, r_cell, r_ent, G * n_rec,
+                                        s_wsum, a.err, p == 0)
+                             : 0;
+    __syncthreads();
+    res_chain(s_cell, s_ent, s_next, ns, n_src);
+    __syncthreads();
+    const bool pts = ns > 0 || nr > 0;
+    // boundary rows that hold sources are published after the injection
+    bool src_up = false, src_dn = false;
+    for (int i = 0; i < ns; ++i) {
+      src_up = src_up || s_cell[i] < W;
+      src_dn = src_dn || s_cell[i] >= (R - 1) * W;
+    }
+    // smem index of a list entry's Ey
+    auto ey_of = [&](int cell, int sh) {
+      const int r = cell / W, x = cell - r * W;
+      return r * rowst + (x >> 5) * (K * 32) + EY + (sh - s0) * 32 + (x & 31);
+    };
+    // first source / receiver entry of this thread, kept in registers
+    int my_src = -1, my_sent = 0, my_snext = -1;
+    if (tid < ns && s_next[tid] >= -1) {
+      my_sent = s_ent[tid];
+      my_src = ey_of(s_cell[tid], my_sent / n_src);
+      my_snext = s_next[tid];
+    }
+    int my_rec = -1, my_rent = 0;
+    if (tid < nr) {
+      my_rent = r_ent[tid];
+      my_rec = ey_of(r_cell[tid], my_rent / n_rec);
+    }
+    // Publish the boundary rows of Ey for `tg`.
+    auto publish = [&](unsigned tg, bool up, bool dn) {
+      for (int x = tid; x < W; x += nthr) {
+        const float *b = blk + (x >> 5) * (K * 32) + (x & 31);
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+          if (k >= ng) break;
+          if (up) ll_store(ll_at(tg, p - 1, 0) + k * W + x, b[EY + k * 32], tg);
+          if (dn) ll_store(ll_at(tg, p, 1) + k * W + x, b[(R - 1) * rowst + EY + k * 32], tg);
+        }
+      }
+    };
+    publish(tag, has_up, has_dn);
+    int64_t slot = (a.t0 + a.ratio - 1) / a.ratio;  // next slot stored, and steps until then
+    int until = a.est || a.cst ? (int)(slot * a.ratio - a.t0) : -1;
+    slot = (slot * S + s0) * g.N;
+    const float *ft = a.f + a.t0 * ((int64_t)S * n_src);
+    float *rt = a.r + a.t0 * ((int64_t)S * n_rec);
+
+    for (int i = 0; i < a.nt; ++i, ++tag) {
+      float fv = 0.f;
+      if (my_src >= 0) fv = __ldg(ft + my_sent);
+      // ------------------------------------------------ H half step
+      {
+        const unsigned long long *const pu0 = ll_at(tag, p - 1, 1);
+        const unsigned long long *const pd0 = ll_at(tag, p, 0);
+        // halo words of a task's columns (first read; see ll_wait)
+        auto first_read = [&](const unsigned long long *p, bool on, unsigned long long (&v)[G]) {
+#pragma unroll
+          for (int k = 0; k < G; ++k) v[k] = on && k < ng ? ll_load(p + k * W) : 0;
+        };
+        auto wait = [&](const unsigned long long *p, bool on, const unsigned long long (&v)[G],
+                        float (&e)[G]) {
+#pragma unroll
+          for (int k = 0; k < G; ++k)
+            e[k] = on && k < ng ? ll_wait(p + k * W, tag, v[k], &s_dead, a.err) : 0.f;
+        };
+        for (int r = gen_r0, gb = gen_b0; r < R;) {  // general tasks
+          const int xb = gb < xb_lo ? gb : gb + n_pl;
+          const int x = xb * 32 + lane, y = ya + r;
+          const bool xin = x >= 1 && x < W;
+          const bool up = has_up && r == 0 && xin, dn = has_dn && r == R - 1 && xin;
+          unsigned long long vu[G], vd[G];
+          first_read(pu0 + x, up, vu);
+          first_read(pd0 + x, dn, vd);
+          const bool hz_ok = xin && x < W - 1 && y >= 1;
+          const bool hx_ok = xin && y >= 1 && y < ny - 1;
+          const bool xs = hz_ok && (x < g.pml_x0 || x >= g.pml_x1h);
+          const bool ys = hx_ok && (y < g.pml_y0 || y >= g.pml_y1h);
+          const int xc = x < g.pml_x0 ? x : x - g.pml_x1h + g.pml_x0;
+          float *const b = blk + r * rowst + xb * (K * 32) + lane;
+          const float *const bn = lane < 31 ? b + 1 : b + K * 32 - 31;
+          float *const mxp = mxh + r * XW + xc;
+          float *const mzp = mzh + ((r + 1) * XB + xb) * (G * 32) + lane;
+          float e0[G], er[G], hx[G], hz[G], e1[G], mx[G], mz[G];
+          const float cqv = b[CQ];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            e0[k] = b[EY + k * 32];
+            er[k] = hz_ok ? bn[EY + k * 32] : 0.f;
+            hx[k] = b[HX + k * 32];
+            hz[k] = b[HZ + k * 32];
+            mx[k] = xs ? mxp[k * R * XW] : 0.f;
+            mz[k] = ys ? mzp[k * 32] : 0.f;
+            e1[k] = r + 1 < R ? b[rowst + EY + k * 32] : 0.f;
+          }
+          if (hz_ok) {
+            float d[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) d[k] = (er[k] - e0[k]) * g.rdx;
+            if (xs) {
+              const ResProf f = pxh[xc];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float mn = f.b * mx[k] + f.a * d[k];
+                mxp[k * R * XW] = mn;
+                d[k] = res_div(d[k], f.k, f.i) + mn;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) b[HZ + k * 32] = hz[k] + cqv * d[k];
+          }
+          if (dn) wait(pd0 + x, dn, vd, e1);
+          if (hx_ok) {
+            float d[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) d[k] = (e1[k] - e0[k]) * g.rdy;
+            if (ys) {
+              const ResProf f = pyh[r];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float mn = f.b * mz[k] + f.a * d[k];
+                mzp[k * 32] = mn;
+                d[k] = res_div(d[k], f.k, f.i) + mn;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) b[HX + k * 32] = hx[k] - cqv * d[k];
+          }
+          if (up) {  // H-x of the row above the slab
+            float eu[G], d[G];
+            // read even where row 0 needs no update: a slab that did not wait for
+            // its neighbour could rewrite a slot before it was read
+            wait(pu0 + x, up, vu, eu);
+            if (ya - 1 >= 1) {
+              float *const h = halo + xb * ((G + 1) * 32) + lane;
+              float *const m = mzh + xb * (G * 32) + lane;
+#pragma unroll
+              for (int k = 0; k < G; ++k) d[k] = (e0[k] - eu[k]) * g.rdy;
+              if (ya - 1 < g.pml_y0 || ya - 1 >= g.pml_y1h) {
+                const ResProf f = pyh[-1];
+#pragma unroll
+                for (int k = 0; k < G; ++k) {
+                  const float mn = f.b * m[k * 32] + f.a * d[k];
+                  m[k * 32] = mn;
+                  d[k] = res_div(d[k], f.k, f.i) + mn;
+                }
+              }
+#pragma unroll
+              for (int k = 0; k < G; ++k) h[k * 32] = h[k * 32] - h[G * 32] * d[k];
+            }
+          }
+          r += gen_dr;
+          gb += gen_db;
+          if (gb >= n_gb) {
+            gb -= n_gb;
+            ++r;
+          }
+        }
+        for (int ch = pl_c0, pb = pl_b0; ch < n_ch;) {  // straight-line tasks
+          const int xb = xb_lo + pb, x = xb * 32 + lane;
+          // the chunk with the slab's first row last: its halo words have arrived
+          const int r0 = (ch + 1 < n_ch ? ch + 1 : 0) * UR, nr_ = min(UR, R - r0);
+          const bool up = has_up && r0 == 0, dn = has_dn && r0 + nr_ == R;
+          unsigned long long vu[G], vd[G];
+          first_read(pu0 + x, up, vu);
+          first_read(pd0 + x, dn, vd);
+          float *const b = blk + r0 * rowst + xb * (K * 32) + lane;
+          const float *const bn = lane < 31 ? b + 1 : b + K * 32 - 31;
+          float e0[G];
+#pragma unroll
+          for (int k = 0; k < G; ++k) e0[k] = b[EY + k * 32];
+          auto rows = [&](auto uu) {
+            constexpr int U = decltype(uu)::value;
+            float c[U], er[U][G], hx[U][G], hz[U][G], e1[U][G];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              c[u] = b[u * rowst + CQ];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                er[u][k] = bn[u * rowst + EY + k * 32];
+                hx[u][k] = b[u * rowst + HX + k * 32];
+                hz[u][k] = b[u * rowst + HZ + k * 32];
+              }
+              if (u + 1 < U || !dn) {
+#pragma unroll
+                for (int k = 0; k < G; ++k) e1[u][k] = b[(u + 1) * rowst + EY + k * 32];
+              }
+            }
+            if (dn) wait(pd0 + x, dn, vd, e1[U - 1]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float e = u ? e1[u ? u - 1 : 0][k] : e0[k];
+                b[u * rowst + HX + k * 32] = hx[u][k] - c[u] * ((e1[u][k] - e) * g.rdy);
+                b[u * rowst + HZ + k * 32] = hz[u][k] + c[u] * ((er[u][k] - e) * g.rdx);
+              }
+            }
+          };
+          res_rows<UR>(nr_, rows);
+          if (up) {
+            float *const h = halo + xb * ((G + 1) * 32) + lane;
+            float eu[G];
+            wait(pu0 + x, up, vu, eu);
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              h[k * 32] = h[k * 32] - h[G * 32] * ((e0[k] - eu[k]) * g.rdy);
+          }
+          ch += pl_dc;
+          pb += pl_db;
+          if (pb >= n_pl) {
+            pb -= n_pl;
+            ++ch;
+          }
+        }
+      }
+      __syncthreads();
+      // ------------------------------------------------ E half step
+      const bool store = until == 0;
+      const bool pub_up = has_up && !src_up && i + 1 < a.nt;
+      const bool pub_dn = has_dn && !src_dn && i + 1 < a.nt;
+      {
+        unsigned long long *const wu0 = ll_at(tag + 1, p - 1, 0), *const wd0 = ll_at(tag + 1, p, 1);
+        Sn *const est = store && a.est ? a.est + slot : nullptr;
+        Sn *const cst = store && a.cst ? a.cst + slot : nullptr;
+        const int bl = lane > 0 ? -1 : 31 - K * 32;  // column x - 1
+        auto put = [&](int r, int x, const float (&en)[G]) {  // boundary rows to the neighbours
+          if (r == 0 && pub_up) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              if (k < ng) ll_store(wu0 + k * W + x, en[k], tag + 1);
+          }
+          if (r == R - 1 && pub_dn) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              if (k < ng) ll_store(wd0 + k * W + x, en[k], tag + 1);
+          }
+        };
+        for (int r = gen_r0, gb = gen_b0; r < R;) {  // general tasks
+          const int xb = gb < xb_lo ? gb : gb + n_pl;
+          const int x = xb * 32 + lane, y = ya + r;
+          const int64_t j = (int64_t)y * W + x;
+          const bool xdom = x >= 1 && x < W, dom = xdom && y >= 1;
+          const bool xs = dom && (x < g.pml_x0 || x >= g.pml_x1);
+          const bool ys = dom && (y < g.pml_y0 || y >= g.pml_y1);
+          const int xc = x < g.pml_x0 ? x : x - g.pml_x1h + g.pml_x0;
+          float *const b = blk + r * rowst + xb * (K * 32) + lane;
+          const float *const hr = halo + xb * ((G + 1) * 32) + lane;
+          float *const mxp = mxe + r * XW + xc, *const mzp = mze + (r * XB + xb) * (G * 32) + lane;
+          const float av = b[CA];
+          const float bv = b[CB];
+          float en[G], dz[G], dy[G], mx[G], mz[G];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            const float hp = r > 0 ? b[HX + k * 32 - rowst] : hr[k * 32];
+            const float hl = xdom ? b[HZ + k * 32 + bl] : 0.f;
+            en[k] = b[EY + k * 32];
+            mx[k] = xs ? mxp[k * R * XW] : 0.f;
+            mz[k] = ys ? mzp[k * 32] : 0.f;
+            dz[k] = (b[HZ + k * 32] - hl) * g.rdx;
+            dy[k] = (b[HX + k * 32] - hp) * g.rdy;
+          }
+          if (dom) {
+            if (xs) {
+              const ResProf f = pxe[xc];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float mn = f.b * mx[k] + f.a * dz[k];
+                mxp[k * R * XW] = mn;
+                dz[k] = res_div(dz[k], f.k, f.i) + mn;
+              }
+            }
+            if (ys) {
+              const ResProf f = pye[r];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float mn = f.b * mz[k] + f.a * dy[k];
+                mzp[k * 32] = mn;
+                dy[k] = res_div(dy[k], f.k, f.i) + mn;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              const float curl = dz[k] - dy[k];
+              if (est && k < ng) store_stream(est + k * g.N + j, Codec<Sn, float>::enc(en[k]));
+              if (cst && k < ng) store_stream(cst + k * g.N + j, Codec<Sn, float>::enc(curl));
+              en[k] = av * en[k] + bv * curl;
+              b[EY + k * 32] = en[k];
+            }
+          }
+          if (xdom) put(r, x, en);
+          r += gen_dr;
+          gb += gen_db;
+          if (gb >= n_gb) {
+            gb -= n_gb;
+            ++r;
+          }
+        }
+        for (int ch = pl_c0, pb = pl_b0; ch < n_ch;) {  // straight-line tasks
+          const int xb = xb_lo + pb, x = xb * 32 + lane;
+          // the slab's first and last rows first: they are published
+          const int r0 = (ch == 0 ? 0 : n_ch - ch) * UR, nr_ = min(UR, R - r0);
+          float *const b = blk + r0 * rowst + xb * (K * 32) + lane;
+          const float *const hr = halo + xb * ((G + 1) * 32) + lane;
+          const int64_t j = (int64_t)(ya + r0) * W + x;
+          auto rows = [&](auto uu) {
+            constexpr int U = decltype(uu)::value;
+            float ca[U], cb[U], hx[U + 1][G], hz[U][G], hl[U][G], e[U][G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) hx[0][k] = r0 > 0 ? b[HX + k * 32 - rowst] : hr[k * 32];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              ca[u] = b[u * rowst + CA];
+              cb[u] = b[u * rowst + CB];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                hx[u + 1][k] = b[u * rowst + HX + k * 32];
+                hz[u][k] = b[u * rowst + HZ + k * 32];
+                hl[u][k] = b[u * rowst + HZ + k * 32 + bl];
+                e[u][k] = b[u * rowst + EY + k * 32];
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float curl =
+                    (hz[u][k] - hl[u][k]) * g.rdx - (hx[u + 1][k] - hx[u][k]) * g.rdy;
+                if (est && k < ng)
+                  store_stream(est + k * g.N + j + u * W, Codec<Sn, float>::enc(e[u][k]));
+                if (cst && k < ng)
+                  store_stream(cst + k * g.N + j + u * W, Codec<Sn, float>::enc(curl));
+                e[u][k] = ca[u] * e[u][k] + cb[u] * curl;
+                b[u * rowst + EY + k * 32] = e[u][k];
+              }
+            }
+            if (r0 == 0) put(0, x, e[0]);
+            if (r0 + U == R && R > 1) put(R - 1, x, e[U - 1]);
+          };
+          res_rows<UR>(nr_, rows);
+          ch += pl_dc;
+          pb += pl_db;
+          if (pb >= n_pl) {
+            pb -= n_pl;
+            ++ch;
+          }
+        }
+      }
+      if (store) {
+        slot += (int64_t)S * g.N;
+        until = a.ratio;
+      }
+      --until;
+      __syncthreads();
+      if (pts) {
+        if (ns > 0) {
+          if (my_src >= 0) {
+            float e = blk[my_src] + fv;
+            for (int k = my_snext; k >= 0; k = res_next(s_next, k)) e = e + __ldg(ft + s_ent[k]);
+            blk[my_src] = e;
+          }
+          for (int k0 = tid + nthr; k0 < ns; k0 += nthr) {
+            if (s_next[k0] < -1) continue;
+            const int o = ey_of(s_cell[k0], s_ent[k0] / n_src);
+            float e = blk[o] + __ldg(ft + s_ent[k0]);
+            for (int k = s_next[k0]; k >= 0; k = res_next(s_next, k)) e = e + __ldg(ft + s_ent[k]);
+            blk[o] = e;
+          }
+          __syncthreads();
+          if ((src_up || src_dn) && i + 1 < a.nt)
+            publish(tag + 1, has_up && src_up, has_dn && src_dn);
+        }
+        if (my_rec >= 0) rt[my_rent] = blk[my_rec];
+        for (int k = tid + nthr; k < nr; k += nthr)
+          rt[r_ent[k]] = blk[ey_of(r_cell[k], r_ent[k] / n_rec)];
+      }
+      ft += (int64_t)S * n_src;
+      rt += (int64_t)S * n_rec;
+    }
+    // ---- state back to the caller
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+      if (k >= ng) break;
+      const int64_t sb = (int64_t)(s0 + k) * g.N;
+      for (int i = tid; i < R * XB * 32; i += nthr) {
+        const int x = i % (XB * 32), r = i / (XB * 32);
+        if (x >= W) continue;
+        const float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        a.ey[j] = b[EY + k * 32];
+        a.hx[j] = b[HX + k * 32];
+        a.hz[j] = b[HZ + k * 32];
+        if (ystrip) {
+          const int o = ((r + 1) * XB + (x >> 5)) * (G * 32) + k * 32 + (x & 31);
+          a.mez[j] = mzh[o];
+          a.mhx[j] = mze[o - XB * G * 32];
+        }
+      }
+      for (int i = tid; i < R * XW; i += nthr) {
+        const int c = i % XW, r = i / XW;
+        const int x = c < g.pml_x0 ? c : c - g.pml_x0 + g.pml_x1h;
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        a.mex[j] = mxh[(k * R + r) * XW + c];
+        a.mhz[j] = mxe[(k * R + r) * XW + c];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------- adjoint
+// The exact adjoint in the same form: per step the adjoint E phase (lambda_H
+// gathers raw terms of cb lambda_Ey), a block barrier, the adjoint H phase
+// (lambda_Ey gathers raw terms of cq lambda_H), receivers' adjoint, source
+// records and the image terms.  The exchange is the boundary rows of
+// lambda_Ey.  A CTA keeps lambda_Hx of the row above its slab and the CPML
+// memories of the rows on both sides, advanced with their owners' operations.
+// The CPML memories have two copies by step parity: a cell's new value is
+// written while its neighbours still read the old one.
+//
+// Images.  A thread sums the image terms of the group's shots (shot order) and
+// adds them to the accumulators of its cell in shared memory.  With one group
+// those start from and end as the gradient itself (step-major, as the per-step
+// kernels); with more each sub-grid accumulates from zero and k_res_combine adds
+// them in order.
+template <typename Sn> struct ResAdjArgs {
+  TMGeom<float> g;
+  ResPlan pl;
+  const float *ca, *cb, *cq;
+  float *ey, *hx, *hz, *mex, *mez, *mhx, *mhz;  // lambda fields and memories
+  ResPoints src, rec;
+  const float *gr;  // [steps, S, n_rec]
+  float *gf;        // [steps, S, n_src], null: not recorded
+  const Sn *est, *cst;
+  int bg;           // shots of the history: shot s images against shot s % bg
+  float *gca, *gcb; // accumulators (see above); with several groups [Q][N]
+  float kscale;
+  int64_t t1;       // first step handled is t1 - 1
+  int nt, ratio;
+  unsigned long long *ll;
+  int *lists;
+  int *err;
+};
+
+__host__ __device__ inline ResSmem res_adj_smem(int R, int XB, int XW, int G, int K,
+                                                bool ystrip) {
+  ResSmem s = res_smem(0, XB, XW, G, K, false);
+  s.pye = s.pyh + 4 * (R + 2);
+  s.pxh = s.pye + 4 * (R + 2);
+  s.pxe = s.pxh + 4 * XW;
+  s.blk = s.pxe + 4 * XW;
+  s.halo = s.blk + R * XB * K * 32;
+  s.mzh = s.halo + XB * (G + 3) * 32;
+  const int ny = ystrip ? XB * G * 32 : 0;
+  s.mze = s.mzh + 2 * (R + 1) * ny;   // m_ey_z: rows -1 .. R - 1
+  s.mxh = s.mze + 2 * (R + 2) * ny;   // m_hx_z: rows -1 .. R
+  s.mxe = s.mxh + 2 * G * R * XW;
+  s.end = s.mxe + 2 * G * R * XW;
+  return s;
+}
+// Does a slab of the adjoint hold (or border on) y-strip rows?
+__host__ __device__ inline bool res_adj_ystrip(const TMGeom<float> &g, int ya, int yb) {
+  return ya - 1 < g.pml_y0 || yb >= g.pml_y1h;
+}
+
+// Moves the slab's rows of a history towards L2 ahead of their use (16-byte
+// granules inside the slab).
+__device__ __forceinline__ void res_prefetch(const void *p, int64_t bytes) {
+  const uint64_t b = (reinterpret_cast<uint64_t>(p) + 15) & ~uint64_t(15);
+  const uint64_t e = (reinterpret_cast<uint64_t>(p) + (uint64_t)bytes) & ~uint64_t(15);
+  if (e > b)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"((unsigned)(e - b))
+                 : "memory");
+}
+
+template <typename Sn, int G>
+__global__ void __launch_bounds__(kResAdjThreads, 1)
+k_res_adj(const __grid_constant__ ResAdjArgs<Sn> a) {
+  constexpr int K = 3 * G + 5;
+  constexpr int EY = 0, HX = G * 32, HZ = 2 * G * 32, CQ = 3 * G * 32, CA = CQ + 32, CB = CQ + 64;
+  constexpr int GA = 3 * G * 32 + 96, GB = GA + 32;
+  constexpr int UR = G == 1 ? 4 : 2;  // rows in flight of the straight-line path
+  constexpr int HB = (G + 3) * 32, HCQ = G * 32, HCB = HCQ + 32, HCD = HCQ + 64;  // halo row block
+  extern __shared__ __align__(16) float sm[];
+  __shared__ int s_dead;
+  __shared__ int s_wsum[kResAdjThreads / 32];
+  __shared__ unsigned char s_row[kResMaxRows];  // rows that hold receivers
+  const TMGeom<float> &g = a.g;
+  const int W = g.nx, ny = g.ny, S = g.n_shots;
+  const int P = a.pl.P, p = blockIdx.x % P, q = blockIdx.x / P;
+  const int ya = a.pl.row[p], yb = a.pl.row[p + 1], R = yb - ya;
+  const int XB = a.pl.XB, XW = a.pl.XW;
+  const bool ystrip = res_adj_ystrip(g, ya, yb);
+  const ResSmem L = res_adj_smem(R, XB, XW, G, K, ystrip);
+  float *const blk = sm + L.blk, *const halo = sm + L.halo;
+  float *const mzh = sm + L.mzh, *const mze = sm + L.mze;
+  float *const mxh = sm + L.mxh, *const mxe = sm + L.mxe;
+  ResProf *const pyh = reinterpret_cast<ResProf *>(sm + L.pyh) + 1;  // [-1]: the row above
+  ResProf *const pye = reinterpret_cast<ResProf *>(sm + L.pye) + 1;
+  ResProf *const pxh = reinterpret_cast<ResProf *>(sm + L.pxh);
+  ResProf *const pxe = reinterpret_cast<ResProf *>(sm + L.pxe);
+  const int xcopy = G * R * XW;  // second copies of the memories
+  const int yst = XB * G * 32;   // row step of the y memories
+  const int hcopy = (R + 1) * yst, ecopy = (R + 2) * yst;
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int rowst = XB * K * 32;
+  const bool has_up = p > 0, has_dn = p + 1 < P;
+  const bool plain = !ystrip && ya >= 2 && yb < ny;  // tasks: see k_res_fwd
+  const int xb_lo = plain ? min(XB, (max(g.pml_x0, 1) + 32) / 32) : XB;
+  const int xb_hi = plain ? max(xb_lo, min(g.pml_x1h, W - 1) / 32) : XB;
+  const int n_pl = xb_hi - xb_lo, n_gb = XB - n_pl, n_gen = n_gb * R;
+  const int nwarps = nthr >> 5;
+  const int gen_r0 = n_gb ? warp / n_gb : 0, gen_b0 = n_gb ? warp - gen_r0 * n_gb : 0;
+  const int gen_dr = n_gb ? nwarps / n_gb : 0, gen_db = n_gb ? nwarps - gen_dr * n_gb : 0;
+  const int pl_t0 = warp >= n_gen ? warp - n_gen
+                                  : (nwarps - (n_gen - warp) % nwarps) % nwarps;
+  const int n_ch = (R + UR - 1) / UR;
+  const int pl_c0 = n_pl ? pl_t0 / n_pl : n_ch, pl_b0 = n_pl ? pl_t0 - pl_c0 * n_pl : 0;
+  const int pl_dc = n_pl ? nwarps / n_pl : 0, pl_db = n_pl ? nwarps - pl_dc * n_pl : 0;
+  const int64_t ll_par = (int64_t)a.pl.Q * (P - 1) * 2 * G * W;
+  unsigned long long *const ll_q = a.ll + (int64_t)q * (P - 1) * 2 * G * W;
+  auto ll_at = [&](unsigned tag, int b, int dir) {
+    return ll_q + (tag & 1) * ll_par + ((int64_t)b * 2 + dir) * G * W;
+  };
+  const int n_src = a.src.n, n_rec = a.rec.n;
+  int *const ls = a.lists + (int64_t)blockIdx.x * G * (2 * n_src + 3 * n_rec);
+  int *const r_cell = ls, *const r_ent = r_cell + G * n_rec, *const r_next = r_ent + G * n_rec;
+  int *const s_cell = r_next + G * n_rec, *const s_ent = s_cell + G * n_src;
+  const bool many = a.pl.n_groups > 1;
+  float *const gca = a.gca ? a.gca + (many ? (int64_t)q * g.N : 0) : nullptr;
+  float *const gcb = a.gcb ? a.gcb + (many ? (int64_t)q * g.N : 0) : nullptr;
+  if (tid == 0) s_dead = 0;
+  res_profiles(g, pyh - 1, pye - 1, pxh, pxe, ya, R, XW);
+
+  for (int i = tid; i < R * XB * 32; i += nthr) {
+    const int x = i % (XB * 32), r = i / (XB * 32);
+    float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+    const int64_t j = (int64_t)(ya + r) * W + x;
+    const bool in = x < W;
+    b[CQ] = in ? __ldg(a.cq + j) : 0.f;
+    b[CA] = in ? __ldg(a.ca + j) : 0.f;
+    b[CB] = in ? __ldg(a.cb + j) : 0.f;
+    // one group: continue the caller's gradient; several: from zero
+    b[GA] = (in && gca && !many) ? gca[j] : 0.f;
+    b[GB] = (in && gcb && !many) ? gcb[j] : 0.f;
+  }
+  for (int x = tid; x < XB * 32; x += nthr) {
+    float *h = halo + (x >> 5) * HB + (x & 31);
+    const bool in = x < W;
+    h[HCQ] = (has_up && in) ? __ldg(a.cq + (int64_t)(ya - 1) * W + x) : 0.f;
+    h[HCB] = (has_up && in) ? __ldg(a.cb + (int64_t)(ya - 1) * W + x) : 0.f;
+    h[HCD] = (has_dn && in) ? __ldg(a.cb + (int64_t)yb * W + x) : 0.f;
+  }
+
+  unsigned tag = 1;
+  int cur = 0;  // copy of the memories that is read
+  for (int grp = q; grp < a.pl.n_groups; grp += a.pl.Q) {
+    const int s0 = res_group_begin(grp, a.pl.n_groups, S);
+    const int ng = res_group_begin(grp + 1, a.pl.n_groups, S) - s0;
+    // ---- state of the group
+#pragma unroll 1
+    for (int k = 0; k < G; ++k) {
+      const int64_t sb = (int64_t)(s0 + k) * g.N;
+      const bool on = k < ng;
+      for (int i = tid; i < R * XB * 32; i += nthr) {
+        const int x = i % (XB * 32), r = i / (XB * 32), y = ya + r;
+        float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+        const int64_t j = sb + (int64_t)y * W + x;
+        const bool in = on && x < W;
+        b[EY + k * 32] = in ? a.ey[j] : 0.f;
+        b[HX + k * 32] = in ? a.hx[j] : 0.f;
+        b[HZ + k * 32] = in ? a.hz[j] : 0.f;
+        // memories: strips are kept, cells outside them are cleared
+        const bool sh = y < g.pml_y0 || y >= g.pml_y1h, se = y < g.pml_y0 || y >= g.pml_y1;
+        if (ystrip) {
+          const int o = (r + 1) * yst + (x >> 5) * (G * 32) + k * 32 + (x & 31);
+          const float vh = (in && sh) ? a.mez[j] : 0.f, ve = (in && se) ? a.mhx[j] : 0.f;
+          mzh[o] = mzh[o + hcopy] = vh;
+          mze[o] = mze[o + ecopy] = ve;
+        }
+        if (in) {
+          if (!sh) a.mez[j] = 0.f;
+          if (!se) a.mhx[j] = 0.f;
+          if (x >= g.pml_x0 && x < g.pml_x1h) a.mex[j] = 0.f;
+          if (x >= g.pml_x0 && x < g.pml_x1) a.mhz[j] = 0.f;
+        }
+      }
+      for (int x = tid; x < XB * 32; x += nthr) {
+        const bool in = on && x < W;
+        const int64_t j = sb + (int64_t)(ya - 1) * W + x;
+        halo[(x >> 5) * HB + k * 32 + (x & 31)] = (in && has_up) ? a.hx[j] : 0.f;
+        if (ystrip) {
+          const int o = (x >> 5) * (G * 32) + k * 32 + (x & 31), yu = ya - 1;
+          const bool sh = yu < g.pml_y0 || yu >= g.pml_y1h, se = yu < g.pml_y0 || yu >= g.pml_y1;
+          const bool sd = yb < g.pml_y0 || yb >= g.pml_y1;
+          const float vh = (in && has_up && sh) ? a.mez[j] : 0.f;
+          const float ve = (in && has_up && se) ? a.mhx[j] : 0.f;
+          const float vd = (in && has_dn && sd) ? a.mhx[sb + (int64_t)yb * W + x] : 0.f;
+          mzh[o] = mzh[o + hcopy] = vh;
+          mze[o] = mze[o + ecopy] = ve;
+          mze[(R + 1) * yst + o] = mze[(R + 1) * yst + o + ecopy] = vd;
+        }
+      }
+      for (int i = tid; i < R * XW; i += nthr) {
+        const int c = i % XW, r = i / XW;
+        const int x = c < g.pml_x0 ? c : c - g.pml_x0 + g.pml_x1h;
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        const int o = (k * R + r) * XW + c;
+        const bool se = x < g.pml_x0 || x >= g.pml_x1;
+        const float vh = on ? a.mex[j] : 0.f, ve = (on && se) ? a.mhz[j] : 0.f;
+        mxh[o] = mxh[o + xcopy] = vh;
+        mxe[o] = mxe[o + xcopy] = ve;
+      }
+    }
+    // ---- point lists of the group
+    const int nr = n_rec > 0 ? res_list(a.rec, s0, ng, ya, yb, W, g.N, r_cell, r_ent, G * n_rec,
+                                        s_wsum, a.err, p == 0)
+                             : 0;
+    const int ns = n_src > 0 ? res_list(a.src, s0, ng, ya, yb, W, g.N, s_cell, s_ent, G * n_src,
+                                        s_wsum, a.err, p == 0)
+                             : 0;
+    for (int i = tid; i < R; i += nthr) s_row[i] = 0;
+    __syncthreads();
+    res_chain(r_cell, r_ent, r_next, nr, n_rec);
+    for (int i = tid; i < nr; i += nthr) s_row[r_cell[i] / W] = 1;
+    __syncthreads();
+    const bool pts = ns > 0 || nr > 0;
+    bool rec_up = false, rec_dn = false;  // boundary rows published after the injection
+    for (int i = 0; i < nr; ++i) {
+      rec_up = rec_up || r_cell[i] < W;
+      rec_dn = rec_dn || r_cell[i] >= (R - 1) * W;
+    }
+    auto ey_of = [&](int cell, int sh) {
+      const int r = cell / W, x = cell - r * W;
+      return r * rowst + (x >> 5) * (K * 32) + EY + (sh - s0) * 32 + (x & 31);
+    };
+    int my_rec = -1, my_rent = 0, my_rnext = -1;
+    if (tid < nr && r_next[tid] >= -1) {
+      my_rent = r_ent[tid];
+      my_rec = ey_of(r_cell[tid], my_rent / n_rec);
+      my_rnext = r_next[tid];
+    }
+    auto publish = [&](unsigned tg, bool up, bool dn) {
+      for (int x = tid; x < W; x += nthr) {
+        const float *b = blk + (x >> 5) * (K * 32) + (x & 31);
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+          if (k >= ng) break;
+          if (up) ll_store(ll_at(tg, p - 1, 0) + k * W + x, b[EY + k * 32], tg);
+          if (dn) ll_store(ll_at(tg, p, 1) + k * W + x, b[(R - 1) * rowst + EY + k * 32], tg);
+        }
+      }
+    };
+    publish(tag, has_up, has_dn);
+    // Histories: slot of the next imaged step at or below the current one, and
+    // the steps until then.
+    const bool any_img = a.est || a.cst;
+    const int64_t sstep = (int64_t)a.bg * g.N;
+    int64_t slot = (a.t1 - 1) / a.ratio;
+    int until = any_img ? (int)(a.t1 - 1 - slot * a.ratio) : -1;
+    int left = (int)(slot - (a.t1 - a.nt + a.ratio - 1) / a.ratio);  // imaged steps after it
+    slot *= sstep;
+    int64_t hoff[G];  // shot offsets in a slot
+#pragma unroll
+    for (int k = 0; k < G; ++k) hoff[k] = (int64_t)((s0 + min(k, ng - 1)) % a.bg) * g.N;
+    const int64_t slab = (int64_t)ya * W;
+    auto prefetch = [&](int64_t o) {  // this slab's rows of the slot at o
+      if (tid < 2 * ng) {
+        const Sn *h = tid & 1 ? a.cst : a.est;
+        const int64_t sh = (int64_t)((s0 + (tid >> 1)) % a.bg) * g.N;
+        if (h) res_prefetch(h + o + sh + slab, (int64_t)R * W * (int64_t)sizeof(Sn));
+      }
+    };
+    if (any_img && left >= 0) prefetch(slot);
+    const float *grt = a.gr + (a.t1 - 1) * ((int64_t)S * n_rec);
+    float *gft = a.gf ? a.gf + (a.t1 - 1) * ((int64_t)S * n_src) : nullptr;
+
+    for (int i = 0; i < a.nt; ++i, ++tag, cur ^= 1) {
+      float gv = 0.f;
+      if (my_rec >= 0) gv = __ldg(grt + my_rent);
+      const bool img = until == 0;
+      if (img && left > 0) prefetch(slot - sstep);
+      // ------------------------------------------------ adjoint E phase
+      {
+        const float *const mxe_c = mxe + cur * xcopy, *const mze_c = mze + cur * ecopy;
+        float *const mxe_n = mxe + (cur ^ 1) * xcopy, *const mze_n = mze + (cur ^ 1) * ecopy;
+        const unsigned long long *const pu0 = ll_at(tag, p - 1, 1);
+        const unsigned long long *const pd0 = ll_at(tag, p, 0);
+        auto first_read = [&](const unsigned long long *p, bool on, unsigned long long (&v)[G]) {
+#pragma unroll
+          for (int k = 0; k < G; ++k) v[k] = on && k < ng ? ll_load(p + k * W) : 0;
+        };
+        auto wait = [&](const unsigned long long *p, bool on, const unsigned long long (&v)[G],
+                        float (&e)[G]) {
+#pragma unroll
+          for (int k = 0; k < G; ++k)
+            e[k] = on && k < ng ? ll_wait(p + k * W, tag, v[k], &s_dead, a.err) : 0.f;
+        };
+        // raw y terms of local row r (-1 .. R) from q = cb lambda; mo: the row's
+        // memory; the new memory is written where this task advances it
+        auto raw_y = [&](int r, int mo, bool write, const float (&q)[G], float (&v)[G]) {
+          const int y = ya + r;
+          if (y >= g.pml_y0 && y < g.pml_y1) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) v[k] = -q[k];
+            return;
+          }
+          const ResProf f = pye[r];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            const float mn = f.b * mze_c[mo + k * 32] - q[k];
+            if (write) mze_n[mo + k * 32] = mn;
+            v[k] = f.a * mn - res_div(q[k], f.k, f.i);
+          }
+        };
+        for (int r = gen_r0, gb = gen_b0; r < R;) {  // general tasks
+          const int xb = gb < xb_lo ? gb : gb + n_pl;
+          const int x = xb * 32 + lane, y = ya + r;
+          const bool xin = x >= 1 && x < W, dom = xin && y >= 1;
+          const bool up = has_up && r == 0 && xin, dn = has_dn && r == R - 1 && xin;
+          unsigned long long vu[G], vd[G];
+          first_read(pu0 + x, up, vu);
+          first_read(pd0 + x, dn, vd);
+          const int xr = x + 1;
+          const bool xr_dom = dom && xr < W;
+          const bool xs = dom && (x < g.pml_x0 || x >= g.pml_x1);
+          const bool xsr = xr_dom && (xr < g.pml_x0 || xr >= g.pml_x1);
+          const int xc = x < g.pml_x0 ? x : x - g.pml_x1h + g.pml_x0;
+          const int xcr = xr < g.pml_x0 ? xr : xr - g.pml_x1h + g.pml_x0;
+          float *const b = blk + r * rowst + xb * (K * 32) + lane;
+          const float *const bn = lane < 31 ? b + 1 : b + K * 32 - 31;
+          const float *const hr = halo + xb * HB + lane;
+          const int ym = (r + 1) * yst + xb * (G * 32) + lane;  // the row's m_hx_z
+          const float cb = b[CB];
+          const float cr = xr_dom ? bn[CB] : 0.f;
+          const float cn = r + 1 < R ? b[rowst + CB] : hr[HCD];
+          float q[G], ln[G], rx[G], rxr[G], ry[G], rn[G];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            q[k] = cb * b[EY + k * 32];
+            rx[k] = q[k];
+            rxr[k] = xr_dom ? cr * bn[EY + k * 32] : 0.f;
+            ln[k] = r + 1 < R ? b[rowst + EY + k * 32] : 0.f;
+            ry[k] = rn[k] = 0.f;
+          }
+          if (dom) raw_y(r, ym, true, q, ry);
+          if (xs) {
+            const ResProf f = pxe[xc];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              const int o = (k * R + r) * XW + xc;
+              const float mn = f.b * mxe_c[o] + q[k];
+              mxe_n[o] = mn;
+              rx[k] = f.a * mn + res_div(q[k], f.k, f.i);
+            }
+          }
+          if (xsr) {
+            const ResProf f = pxe[xcr];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              const float mn = f.b * mxe_c[(k * R + r) * XW + xcr] + rxr[k];
+              rxr[k] = f.a * mn + res_div(rxr[k], f.k, f.i);
+            }
+          }
+          if (dom) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              b[HZ + k * 32] = b[HZ + k * 32] + (rx[k] - rxr[k]) * g.rdx;
+          }
+          if (dn) wait(pd0 + x, dn, vd, ln);
+          if (xin && y + 1 < ny) {
+            float qn[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) qn[k] = cn * ln[k];
+            raw_y(r + 1, ym + yst, r + 1 == R, qn, rn);
+          }
+          if (dom) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              b[HX + k * 32] = b[HX + k * 32] + (ry[k] - rn[k]) * g.rdy;
+          }
+          if (up) {  // lambda_Hx of the row above the slab
+            float lu[G], ru[G];
+            wait(pu0 + x, up, vu, lu);  // (read even for row 0: see k_res_fwd)
+            if (ya - 1 >= 1) {
+              float *const h = halo + xb * HB + lane;
+#pragma unroll
+              for (int k = 0; k < G; ++k) lu[k] = h[HCB] * lu[k];
+              raw_y(-1, xb * (G * 32) + lane, true, lu, ru);
+#pragma unroll
+              for (int k = 0; k < G; ++k) h[k * 32] = h[k * 32] + (ru[k] - ry[k]) * g.rdy;
+            }
+          }
+          r += gen_dr;
+          gb += gen_db;
+          if (gb >= n_gb) {
+            gb -= n_gb;
+            ++r;
+          }
+        }
+        for (int ch = pl_c0, pb = pl_b0; ch < n_ch;) {  // straight-line tasks
+          const int xb = xb_lo + pb, x = xb * 32 + lane;
+          const int r0 = (ch + 1 < n_ch ? ch + 1 : 0) * UR, nr_ = min(UR, R - r0);
+          const bool up = has_up && r0 == 0, dn = has_dn && r0 + nr_ == R;
+          unsigned long long vu[G], vd[G];
+          first_read(pu0 + x, up, vu);
+          first_read(pd0 + x, dn, vd);
+          float *const b = blk + r0 * rowst + xb * (K * 32) + lane;
+          const float *const bn = lane < 31 ? b + 1 : b + K * 32 - 31;
+          float qf[G];
+          {
+            const float c = b[CB];
+#pragma unroll
+            for (int k = 0; k < G; ++k) qf[k] = c * b[EY + k * 32];
+          }
+          auto rows = [&](auto uu) {
+            constexpr int U = decltype(uu)::value;
+            float cn[U], cr[U], ln[U][G], lr[U][G], hx[U][G], hz[U][G], q[G];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              cr[u] = bn[u * rowst + CB];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                lr[u][k] = bn[u * rowst + EY + k * 32];
+                hx[u][k] = b[u * rowst + HX + k * 32];
+                hz[u][k] = b[u * rowst + HZ + k * 32];
+              }
+              if (u + 1 < U || !dn) {
+                cn[u] = b[(u + 1) * rowst + CB];
+#pragma unroll
+                for (int k = 0; k < G; ++k) ln[u][k] = b[(u + 1) * rowst + EY + k * 32];
+              }
+            }
+            if (dn) {
+              cn[U - 1] = halo[xb * HB + lane + HCD];
+              wait(pd0 + x, dn, vd, ln[U - 1]);
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) q[k] = qf[k];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float qn = cn[u] * ln[u][k], qr = cr[u] * lr[u][k];
+                b[u * rowst + HZ + k * 32] = hz[u][k] + (q[k] - qr) * g.rdx;
+                b[u * rowst + HX + k * 32] = hx[u][k] + ((-q[k]) - (-qn)) * g.rdy;
+                q[k] = qn;
+              }
+            }
+          };
+          res_rows<UR>(nr_, rows);
+          if (up) {
+            float *const h = halo + xb * HB + lane;
+            float lu[G];
+            wait(pu0 + x, up, vu, lu);
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              h[k * 32] = h[k * 32] + ((-(h[HCB] * lu[k])) - (-qf[k])) * g.rdy;
+          }
+          ch += pl_dc;
+          pb += pl_db;
+          if (pb >= n_pl) {
+            pb -= n_pl;
+            ++ch;
+          }
+        }
+      }
+      // ------------------------------------------------ adjoint H phase
+      const Sn *const est = img && a.est ? a.est + slot : nullptr;
+      const Sn *const cst = img && a.cst ? a.cst + slot : nullptr;
+      auto load_hist = [&](int64_t j, Sn (&ev)[G], Sn (&cv)[G]) {
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+          ev[k] = est ? load_stream(est + hoff[k] + j) : Sn(0.f);
+          cv[k] = cst ? load_stream(cst + hoff[k] + j) : Sn(0.f);
+        }
+      };
+      // image terms of one cell: lambda values v of the group's shots
+      auto image = [&](float *b, const float (&v)[G], const Sn (&ev)[G],
+                       const Sn (&cv)[G]) {
+        if (est) {
+          float s = 0.f;
+#pragma unroll
+          for (int k = 0; k < G; ++k)
+            if (k < ng) s = s + v[k] * Codec<Sn, float>::dec(ev[k]) * a.kscale;
+          b[GA] = b[GA] + s;
+        }
+        if (cst) {
+          float s = 0.f;
+#pragma unroll
+          for (int k = 0; k < G; ++k)
+            if (k < ng) s = s + v[k] * Codec<Sn, float>::dec(cv[k]) * a.kscale;
+          b[GB] = b[GB] + s;
+        }
+      };
+      const bool pub_up = has_up && !rec_up && i + 1 < a.nt;
+      const bool pub_dn = has_dn && !rec_dn && i + 1 < a.nt;
+      __syncthreads();
+      {
+        const float *const mxh_c = mxh + cur * xcopy, *const mzh_c = mzh + cur * hcopy;
+        float *const mxh_n = mxh + (cur ^ 1) * xcopy, *const mzh_n = mzh + (cur ^ 1) * hcopy;
+        unsigned long long *const wu0 = ll_at(tag + 1, p - 1, 0), *const wd0 = ll_at(tag + 1, p, 1);
+        const int bl = lane > 0 ? -1 : 31 - K * 32;  // column x - 1
+        auto put = [&](int r, int x, const float (&v)[G]) {
+          if (r == 0 && pub_up) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              if (k < ng) ll_store(wu0 + k * W + x, v[k], tag + 1);
+          }
+          if (r == R - 1 && pub_dn) {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+              if (k < ng) ll_store(wd0 + k * W + x, v[k], tag + 1);
+          }
+        };
+        // raw z terms of local row r (-1 .. R - 1) from q = -cq lambda_Hx
+        auto raw_z = [&](int r, int mo, const float (&q)[G], float (&v)[G], bool write) {
+          const int y = ya + r;
+          if (y >= g.pml_y0 && y < g.pml_y1h) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) v[k] = q[k];
+            return;
+          }
+          const ResProf f = pyh[r];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            const float mn = f.b * mzh_c[mo + k * 32] + q[k];
+            if (write) mzh_n[mo + k * 32] = mn;
+            v[k] = f.a * mn + res_div(q[k], f.k, f.i);
+          }
+        };
+        for (int r = gen_r0, gb = gen_b0; r < R;) {  // general tasks
+          const int xb = gb < xb_lo ? gb : gb + n_pl;
+          const int x = xb * 32 + lane, y = ya + r;
+          const int64_t j = (int64_t)y * W + x;
+          const bool xdom = x >= 1 && x < W, dom = xdom && y >= 1;
+          Sn ev[G], cv[G];
+          if (img && dom) load_hist(j, ev, cv);
+          const int xl = x - 1;
+          const bool rx_ok = dom && x < W - 1, rxl_ok = dom && xl >= 1 && xl < W - 1;
+          const bool xs = rx_ok && (x < g.pml_x0 || x >= g.pml_x1h);
+          const bool xsl = rxl_ok && (xl < g.pml_x0 || xl >= g.pml_x1h);
+          const int xc = x < g.pml_x0 ? x : x - g.pml_x1h + g.pml_x0;
+          const int xcl = xl < g.pml_x0 ? xl : xl - g.pml_x1h + g.pml_x0;
+          float *const b = blk + r * rowst + xb * (K * 32) + lane;
+          const float *const hr = halo + xb * HB + lane;
+          const int ym = (r + 1) * yst + xb * (G * 32) + lane;  // the row's m_ey_z
+          const bool zok = dom && y < ny - 1, zpok = xdom && y - 1 >= 1 && y - 1 < ny - 1;
+          const float cq = b[CQ];
+          const float ca = b[CA];
+          const float cl = rxl_ok ? b[CQ + bl] : 0.f;
+          const float cp = r > 0 ? b[CQ - rowst] : hr[HCQ];
+          float v[G], zp[G], z[G], rzp[G], rz[G], rx[G], rxl[G];
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            v[k] = b[EY + k * 32];
+            zp[k] = -cp * (r > 0 ? b[HX + k * 32 - rowst] : hr[k * 32]);
+            z[k] = -cq * b[HX + k * 32];
+            rx[k] = rx_ok ? cq * b[HZ + k * 32] : 0.f;
+            rxl[k] = rxl_ok ? cl * b[HZ + k * 32 + bl] : 0.f;
+            rzp[k] = rz[k] = 0.f;
+          }
+          // the slab's own copy of the row above is advanced with row 0
+          if (zpok) raw_z(r - 1, ym - yst, zp, rzp, r == 0);
+          if (zok) raw_z(r, ym, z, rz, true);
+          if (xs) {
+            const ResProf f = pxh[xc];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              const int o = (k * R + r) * XW + xc;
+              const float mn = f.b * mxh_c[o] + rx[k];
+              mxh_n[o] = mn;
+              rx[k] = f.a * mn + res_div(rx[k], f.k, f.i);
+            }
+          }
+          if (xsl) {
+            const ResProf f = pxh[xcl];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              const float mn = f.b * mxh_c[(k * R + r) * XW + xcl] + rxl[k];
+              rxl[k] = f.a * mn + res_div(rxl[k], f.k, f.i);
+            }
+          }
+          if (dom) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+              v[k] = ca * v[k];
+              v[k] = v[k] + ((rzp[k] - rz[k]) * g.rdy + (rxl[k] - rx[k]) * g.rdx);
+              b[EY + k * 32] = v[k];
+            }
+          }
+          if (xdom) put(r, x, v);
+          if (img && dom && !(nr > 0 && s_row[r])) image(b, v, ev, cv);
+          r += gen_dr;
+          gb += gen_db;
+          if (gb >= n_gb) {
+            gb -= n_gb;
+            ++r;
+          }
+        }
+        for (int ch = pl_c0, pb = pl_b0; ch < n_ch;) {  // straight-line tasks
+          const int xb = xb_lo + pb, x = xb * 32 + lane;
+          const int r0 = (ch == 0 ? 0 : n_ch - ch) * UR, nr_ = min(UR, R - r0);
+          float *const b = blk + r0 * rowst + xb * (K * 32) + lane;
+          const float *const hr = halo + xb * HB + lane;
+          const int64_t j = (int64_t)(ya + r0) * W + x;
+          auto rows = [&](auto uu) {
+            constexpr int U = decltype(uu)::value;
+            Sn ev[U][G], cv[U][G];
+#pragma unroll
+            for (int u = 0; u < U; ++u) load_hist(j + u * W, ev[u], cv[u]);
+            float cq[U + 1], cl[U], ca[U], hx[U + 1][G], hz[U][G], hl[U][G], v[U][G];
+            if (r0 > 0) {
+              cq[0] = b[CQ - rowst];
+#pragma unroll
+              for (int k = 0; k < G; ++k) hx[0][k] = b[HX + k * 32 - rowst];
+            } else {
+              cq[0] = hr[HCQ];
+#pragma unroll
+              for (int k = 0; k < G; ++k) hx[0][k] = hr[k * 32];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              cq[u + 1] = b[u * rowst + CQ];
+              cl[u] = b[u * rowst + CQ + bl];
+              ca[u] = b[u * rowst + CA];
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                hx[u + 1][k] = b[u * rowst + HX + k * 32];
+                hz[u][k] = b[u * rowst + HZ + k * 32];
+                hl[u][k] = b[u * rowst + HZ + k * 32 + bl];
+                v[u][k] = b[u * rowst + EY + k * 32];
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+              for (int k = 0; k < G; ++k) {
+                const float rz0 = -cq[u] * hx[u][k], rz1 = -cq[u + 1] * hx[u + 1][k];
+                const float rx = cq[u + 1] * hz[u][k], rxl = cl[u] * hl[u][k];
+                v[u][k] = ca[u] * v[u][k];
+                v[u][k] = v[u][k] + ((rz0 - rz1) * g.rdy + (rxl - rx) * g.rdx);
+                b[u * rowst + EY + k * 32] = v[u][k];
+              }
+            }
+            if (r0 == 0) put(0, x, v[0]);
+            if (r0 + U == R && R > 1) put(R - 1, x, v[U - 1]);
+            if (img) {
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                if (!(nr > 0 && s_row[r0 + u]))
+                  image(b + u * rowst, v[u], ev[u], cv[u]);
+            }
+          };
+          res_rows<UR>(nr_, rows);
+          ch += pl_dc;
+          pb += pl_db;
+          if (pb >= n_pl) {
+            pb -= n_pl;
+            ++ch;
+          }
+        }
+      }
+      __syncthreads();
+      if (pts) {
+        if (nr > 0) {
+          if (my_rec >= 0) {
+            float e = blk[my_rec] + gv;
+            for (int k = my_rnext; k >= 0; k = res_next(r_next, k)) e = e + __ldg(grt + r_ent[k]);
+            blk[my_rec] = e;
+          }
+          for (int k0 = tid + nthr; k0 < nr; k0 += nthr) {
+            if (r_next[k0] < -1) continue;
+            const int o = ey_of(r_cell[k0], r_ent[k0] / n_rec);
+            float e = blk[o] + __ldg(grt + r_ent[k0]);
+            for (int k = r_next[k0]; k >= 0; k = res_next(r_next, k)) e = e + __ldg(grt + r_ent[k]);
+            blk[o] = e;
+          }
+          __syncthreads();
+          if ((rec_up || rec_dn) && i + 1 < a.nt)
+            publish(tag + 1, has_up && rec_up, has_dn && rec_dn);
+        }
+        if (gft)
+          for (int k = tid; k < ns; k += nthr)
+            gft[s_ent[k]] = blk[ey_of(s_cell[k], s_ent[k] / n_src)];
+        if (img && nr > 0) {  // rows that hold receivers: images of the finished values
+          for (int r = 0; r < R; ++r) {
+            if (!s_row[r] || ya + r < 1) continue;
+            for (int xb = warp; xb < XB; xb += nthr >> 5) {
+              const int x = xb * 32 + lane;
+              if (x < 1 || x >= W) continue;
+              const int64_t j = (int64_t)(ya + r) * W + x;
+              float *b = blk + r * rowst + xb * (K * 32) + lane;
+              Sn ev[G], cv[G];
+              load_hist(j, ev, cv);
+              float v[G];
+#pragma unroll
+              for (int k = 0; k < G; ++k) v[k] = b[EY + k * 32];
+              image(b, v, ev, cv);
+            }
+          }
+        }
+      }
+      if (img) {
+        slot -= sstep;
+        until = left > 0 ? a.ratio : -1;
+        --left;
+      }
+      --until;
+      grt -= (int64_t)S * n_rec;
+      if (gft) gft -= (int64_t)S * n_src;
+    }
+    // ---- state back to the caller
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < ng; ++k) {
+      const int64_t sb = (int64_t)(s0 + k) * g.N;
+      for (int i = tid; i < R * XB * 32; i += nthr) {
+        const int x = i % (XB * 32), r = i / (XB * 32), y = ya + r;
+        if (x >= W) continue;
+        const float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+        const int64_t j = sb + (int64_t)y * W + x;
+        a.ey[j] = b[EY + k * 32];
+        a.hx[j] = b[HX + k * 32];
+        a.hz[j] = b[HZ + k * 32];
+        if (ystrip) {
+          const int o = (r + 1) * yst + (x >> 5) * (G * 32) + k * 32 + (x & 31);
+          if (y < g.pml_y0 || y >= g.pml_y1h) a.mez[j] = mzh[o + cur * hcopy];
+          if (y < g.pml_y0 || y >= g.pml_y1) a.mhx[j] = mze[o + cur * ecopy];
+        }
+      }
+      for (int i = tid; i < R * XW; i += nthr) {
+        const int c = i % XW, r = i / XW;
+        const int x = c < g.pml_x0 ? c : c - g.pml_x0 + g.pml_x1h;
+        const int64_t j = sb + (int64_t)(ya + r) * W + x;
+        const int o = cur * xcopy + (k * R + r) * XW + c;
+        a.mex[j] = mxh[o];
+        if (x < g.pml_x0 || x >= g.pml_x1) a.mhz[j] = mxe[o];
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < R * XB * 32; i += nthr) {
+    const int x = i % (XB * 32), r = i / (XB * 32);
+    if (x >= W) continue;
+    const float *b = blk + r * rowst + (x >> 5) * (K * 32) + (x & 31);
+    const int64_t j = (int64_t)(ya + r) * W + x;
+    if (gca) gca[j] = b[GA];
+    if (gcb) gcb[j] = b[GB];
+  }
+}
+
+// grad[j] += acc[0][j] + ... + acc[n - 1][j] in order.
+static __global__ void k_res_combine(float *grad, const float *acc, int n, int64_t N) {
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < N;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    float s = acc[j];
+    for (int i = 1; i < n; ++i) s = s + acc[(int64_t)i * N + j];
+    grad[j] = grad[j] + s;
+  }
+}
+
+}  // namespace tb

@@ -1,0 +1,55 @@
+// Host interface of the resident TM2D time loops (tm2d_res.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <cstdint>
+
+#include "tm2d_kernels.cuh"
+
+namespace tb {
+
+enum class ResRun { kNotTaken, kDone, kFailed };
+
+// One forward call (with or without a device snapshot history).  Arrays are
+// the entry points' (include/tide_b200.h); est / cst point at slot 0 of the
+// histories, element float or bf16.
+struct ResFwdCall {
+  TMGeom<float> g;
+  const float *ca, *cb, *cq;
+  float *fields[7];  // ey, hx, hz, m_ey_x, m_ey_z, m_hx_z, m_hz_x
+  const int64_t *src_i, *rec_i;
+  int64_t n_src, n_rec;
+  const float *f;
+  float *r;
+  void *est, *cst;
+  bool bf16;
+  int64_t t0, nt, ratio;
+  cudaStream_t st;
+  int *err;  // device error word
+};
+
+// Runs the call as one cooperative launch when its state fits on chip.
+ResRun res_forward(const ResFwdCall &c);
+
+// One backward call over steps t1 - 1 down to t1 - nt.  fields: lambda_ey, _hx,
+// _hz and the four lambda memories; est / cst: slot 0 of device histories of bg
+// shots per slot (null: that image off).
+struct ResAdjCall {
+  TMGeom<float> g;
+  const float *ca, *cb, *cq;
+  float *fields[7];
+  const int64_t *src_i, *rec_i;
+  int64_t n_src, n_rec;
+  const float *grad_r;
+  float *grad_f;
+  const void *est, *cst;
+  bool bf16;
+  int bg;
+  float *grad_ca, *grad_cb;
+  int64_t t1, nt, ratio;
+  cudaStream_t st;
+  int *err;
+};
+ResRun res_backward(const ResAdjCall &c);
+
+}  // namespace tb
