@@ -177,7 +177,8 @@ bool build_list(const int64_t *idx, int n_per_shot, int n_shots, int64_t N, int 
   const int thr = 256, blk = (n + thr - 1) / thr;
   k_points_count<<<blk, thr, 0, st>>>(idx, n_per_shot, n_shots, N, nx, pt, count);
   k_points_scan<<<1, 1024, 0, st>>>(count, start, n_tiles);
-  k_points_fill<<<blk, thr, 0, st>>>(idx, n_per_shot, n_shots, N, nx, pt, start, cell, ent);
+  const unsigned warp_blk = (unsigned)(((int64_t)n * 32 + thr - 1) / thr);
+  k_points_fill<<<warp_blk, thr, 0, st>>>(idx, n_per_shot, n_shots, N, nx, pt, start, cell, ent);
   if (TB_CUDA(cudaGetLastError())) return false;
   count_launches(3);
   out = PointCSR{start, cell, ent};
