@@ -239,7 +239,11 @@ inline void launch_fwd_e(const Launch<T, ST> &L, cudaStream_t st, const T *ca, c
                          S *c_st, const DebyeArgs<T> &db, const PointScratch &ps, const T *ft,
                          T *rt, const StepShift &sh = StepShift{}) {
   constexpr int NB = Launch<T, ST>::kNarrowBY;
-  if (ST == 2 && db.n_poles == 0 && L.e_by == NB)
+  if (ST == 2 && db.n_poles == 1 && L.e_by != NB) {
+    if constexpr (ST == 2)
+      k2_fwd_e_debye<T, S, kRowsE><<<L.grid_e, L.block, 0, st>>>(
+          L.g, ca, cb, hx, hz, ey, m_hx_z, m_hz_x, e_st, c_st, ps.src, ps.rec, ft, rt, db, sh);
+  } else if (ST == 2 && db.n_poles == 0 && L.e_by == NB)
     k2_fwd_e<T, S, kRowsE, NB><<<L.grid_e_n, dim3(kTileX, NB, 1), 0, st>>>(
         L.g, ca, cb, hx, hz, ey, m_hx_z, m_hz_x, e_st, c_st, ps.src, ps.rec, ft, rt, sh);
   else if (ST == 2 && db.n_poles == 0)

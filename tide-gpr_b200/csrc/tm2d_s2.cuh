@@ -138,14 +138,17 @@ k2_fwd_h(TMGeom<T> g, const T *__restrict__ cq, const T *__restrict__ ey, T *__r
 }
 
 // ---------------------------------------------------------------- forward E
-// Full-grid tiles (32 x 8R) so point entries outside the domain are served.
-template <typename T, typename S, int R, int BY = kBlockY, typename TL>
+// Full-grid tiles (32 x 8R) so point entries outside the domain are served.  DB:
+// a medium with one Debye pole (db), whose polarisation is read, stored and
+// advanced with the cell.
+template <typename T, typename S, int R, int BY = kBlockY, bool DB = false, typename TL>
 __device__ __forceinline__ void fwd_e_tile(
     const TL tl, const TMGeom<T> &g,
     const T *__restrict__ ca, const T *__restrict__ cb, const T *__restrict__ hx,
     const T *__restrict__ hz, T *__restrict__ ey, T *__restrict__ m_hx_z,
     T *__restrict__ m_hz_x, S *__restrict__ ey_store, S *__restrict__ curl_store,
-    PointCSR src, PointCSR rec, const T *__restrict__ f_t, T *__restrict__ r_t) {
+    PointCSR src, PointCSR rec, const T *__restrict__ f_t, T *__restrict__ r_t,
+    const DebyeArgs<T> &db = DebyeArgs<T>{}) {
   const int nx = g.nx, ny = g.ny;
   const int x = tl.x() * kTileX + threadIdx.x;
   const int y0 = (tl.y() * BY + threadIdx.y) * R;
@@ -159,13 +162,22 @@ __device__ __forceinline__ void fwd_e_tile(
   if (g.cb_b) cb += base;
   if (ey_store) ey_store += base;
   if (curl_store) curl_store += base;
+  T *const pol = DB ? db.pol + base : nullptr;
+  S *const pol_st = DB && db.pol_st ? static_cast<S *>(db.pol_st) + base : nullptr;
+  S *const esum_st = DB && db.esum_st ? static_cast<S *>(db.esum_st) + base : nullptr;
+  // polarisation after the cell's new Ey (points applied)
+  auto advance_pol = [&](int j, T pv, T da, T dbv, T e, T e_old) {
+    const T e_sum = e + e_old;
+    if (esum_st) store_stream(esum_st + j, Codec<S, T>::enc(e_sum));
+    pol[j] = da * pv + dbv * e_sum;
+  };
   const int j0 = y0 * nx + x;
   {
     // Interior tile (block-uniform): no strip cell, every cell in the domain.
     const int tx0 = tl.x() * kTileX, ty0 = tl.y() * BY * R;
     if (tx0 >= g.pml_x0 && tx0 + kTileX <= g.pml_x1 && ty0 >= g.pml_y0 &&
         ty0 + BY * R <= g.pml_y1) {
-      T vx[R + 1], vz[R], vzl[R], eo[R], a[R], b[R];
+      T vx[R + 1], vz[R], vzl[R], eo[R], a[R], b[R], pv[R], pc[R], da[R], dv[R];
 #pragma unroll
       for (int r = 0; r <= R; ++r) vx[r] = ldg(hx + j0 + (r - 1) * nx);
 #pragma unroll
@@ -176,6 +188,12 @@ __device__ __forceinline__ void fwd_e_tile(
         vzl[r] = ldg(hz + j - 1);
         a[r] = ldg(ca + j);
         b[r] = ldg(cb + j);
+        if (DB) {
+          pv[r] = pol[j];
+          pc[r] = ldg(db.cp + j);
+          da[r] = ldg(db.a + j);
+          dv[r] = ldg(db.b + j);
+        }
       }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -184,8 +202,13 @@ __device__ __forceinline__ void fwd_e_tile(
         if (ey_store) store_stream(ey_store + j, Codec<S, T>::enc(eo[r]));
         if (curl_store) store_stream(curl_store + j, Codec<S, T>::enc(curl));
         T e = a[r] * eo[r] + b[r] * curl;
+        if (DB) {
+          if (pol_st) store_stream(pol_st + j, Codec<S, T>::enc(pv[r]));
+          e = e + ((T)0 + pc[r] * pv[r]);
+        }
         if (pts) e = point_accumulate(src, tile, j, f_t, e);
         ey[j] = e;
+        if (DB) advance_pol(j, pv[r], da[r], dv[r], e, eo[r]);
         if (pts) point_record(rec, tile, j, r_t, e);
       }
       return;
@@ -195,6 +218,7 @@ __device__ __forceinline__ void fwd_e_tile(
   const bool xs = xdom && (x < g.pml_x0 || x >= g.pml_x1);
   // ---- loads
   T vx[R + 1], vz[R], vzl[R], eo[R], a[R], b[R], mz[R], mx[R], pb[R], pa[R], pk[R];
+  T pv[R], pc[R], da[R], dv[R];
   T qb = 0, qa = 0, qk = 1;
   if (xs) {
     qb = ldg(g.bx + x);
@@ -221,6 +245,12 @@ __device__ __forceinline__ void fwd_e_tile(
     pa[r] = ys ? ldg(g.ay + y) : (T)0;
     pk[r] = ys ? ldg(g.ky + y) : (T)1;
     mx[r] = (dom && xs) ? m_hz_x[j] : (T)0;
+    if (DB && dom) {
+      pv[r] = pol[j];
+      pc[r] = ldg(db.cp + j);
+      da[r] = ldg(db.a + j);
+      dv[r] = ldg(db.b + j);
+    }
   }
   // ---- arithmetic and stores
 #pragma unroll
@@ -246,9 +276,14 @@ __device__ __forceinline__ void fwd_e_tile(
       if (ey_store) store_stream(ey_store + j, Codec<S, T>::enc(e));
       if (curl_store) store_stream(curl_store + j, Codec<S, T>::enc(curl));
       e = a[r] * e + b[r] * curl;
+      if (DB) {
+        if (pol_st) store_stream(pol_st + j, Codec<S, T>::enc(pv[r]));
+        e = e + ((T)0 + pc[r] * pv[r]);
+      }
     }
     if (pts) e = point_accumulate(src, tile, j, f_t, e);
     if (dom || pts) ey[j] = e;
+    if (DB && dom) advance_pol(j, pv[r], da[r], dv[r], e, eo[r]);
     if (pts) point_record(rec, tile, j, r_t, e);
   }
 }
@@ -268,6 +303,25 @@ k2_fwd_e(TMGeom<T> g, const T *__restrict__ ca, const T *__restrict__ cb, const 
   }
   fwd_e_tile<T, S, R, BY>(HwTile(), g, ca, cb, hx, hz, ey, m_hx_z, m_hz_x, ey_store, curl_store,
       src, rec, f_t, r_t);
+}
+
+// One Debye pole (the generic kernel of tm2d_kernels.cuh loads the pole's arrays
+// after the update that waits for them: 829 x 1597, 4 shots, 74 us a step, half the
+// steps storing, against 62 here).
+template <typename T, typename S, int R>
+__global__ void __launch_bounds__(32 * kBlockY)
+k2_fwd_e_debye(TMGeom<T> g, const T *__restrict__ ca, const T *__restrict__ cb,
+               const T *__restrict__ hx, const T *__restrict__ hz, T *__restrict__ ey,
+               T *__restrict__ m_hx_z, T *__restrict__ m_hz_x, S *__restrict__ ey_store,
+               S *__restrict__ curl_store, PointCSR src, PointCSR rec,
+               const T *__restrict__ f_t, T *__restrict__ r_t, DebyeArgs<T> db, StepShift sh) {
+  if (sh.blk) {
+    const int64_t jb = sh.block();
+    f_t = shifted(f_t, sh.src, jb);
+    r_t = shifted(r_t, sh.rec, jb);
+  }
+  fwd_e_tile<T, S, R, kBlockY, true>(HwTile(), g, ca, cb, hx, hz, ey, m_hx_z, m_hz_x, ey_store,
+      curl_store, src, rec, f_t, r_t, db);
 }
 
 // ---------------------------------------------------------------- adjoint E
