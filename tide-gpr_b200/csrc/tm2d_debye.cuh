@@ -49,6 +49,41 @@ k_debye_pre(int ny, int nx, int n_poles, const T *__restrict__ a, const T *__res
   U[i] = u;
 }
 
+// One pole: a thread takes all shots of its cell, four at a time, so that the pole
+// coefficients are read once and the loads of four shots are in flight.  HBM bound
+// (16 B a cell and shot).  One shot a thread, as the general kernel above: 81 us on
+// 829 x 1597, 4 shots, against 21 us here.
+template <typename T, int ST>
+__global__ void __launch_bounds__(256)
+k_debye_pre1(int ny, int nx, int n_shots, const T *__restrict__ a, const T *__restrict__ b,
+             const T *__restrict__ cp, const T *__restrict__ g, T *__restrict__ lpol,
+             T *__restrict__ Uv) {
+  constexpr int U = 4;
+  const int64_t N = (int64_t)ny * nx;
+  int64_t j;
+  if (!debye_cell<ST>(ny, nx, j)) return;
+  const T av = ldg(a + j), bv = ldg(b + j), cv = ldg(cp + j);
+  auto group = [&](auto uu, int s0) {
+    constexpr int V = decltype(uu)::value;
+    T lp[V], gv[V];
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      const int64_t i = (int64_t)(s0 + u) * N + j;
+      lp[u] = lpol[i];
+      gv[u] = ldg(g + i);
+    }
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+      const int64_t i = (int64_t)(s0 + u) * N + j;
+      Uv[i] = (T)0 + bv * lp[u];
+      lpol[i] = av * lp[u] + cv * gv[u];
+    }
+  };
+  int s = 0;
+  for (; s + U <= n_shots; s += U) group(std::integral_constant<int, U>(), s);
+  for (; s < n_shots; ++s) group(std::integral_constant<int, 1>(), s);
+}
+
 template <typename T> struct DebyeImages {
   const void *ey_st, *cu_st, *pol_st, *esum_st;  // this step's snapshots (null: none)
   T *grad_ca, *grad_cb, *grad_cp, *grad_a, *grad_b;
@@ -292,8 +327,12 @@ void debye_backward(const TideTMDebye &A) {
                         nxt_hz_x);
     std::swap(cur_hx_z, nxt_hx_z);
     std::swap(cur_hz_x, nxt_hz_x);
-    k_debye_pre<T, ST><<<pgrid, pblk, 0, st>>>((int)A.ny, (int)A.nx, (int)np, da, db, dcp, lam[0],
-                                              lpol, U);
+    if (np == 1)
+      k_debye_pre1<T, ST><<<cgrid, pblk, 0, st>>>((int)A.ny, (int)A.nx, (int)A.n_shots, da, db,
+                                                  dcp, lam[0], lpol, U);
+    else
+      k_debye_pre<T, ST><<<pgrid, pblk, 0, st>>>((int)A.ny, (int)A.nx, (int)np, da, db, dcp,
+                                                 lam[0], lpol, U);
     launch_adj_h<T, ST, T>(L, st, ca, cq, lam[1], lam[2], lam[0], cur_ey_x, cur_ey_z, nxt_ey_x,
                            nxt_ey_z, ps, grad_r ? grad_r + t * rs : nullptr, nullptr, none);
     std::swap(cur_ey_x, nxt_ey_x);
