@@ -301,3 +301,31 @@ def test_high_order_public_api_fp64_vs_reference_golden(cuda_device, stencil):
     (r * w).sum().backward()
     assert rel_l2(eps.grad, torch.from_numpy(hi[f"geps_s{stencil}"])) < 1e-9
     assert rel_l2(sig.grad, torch.from_numpy(hi[f"gsig_s{stencil}"])) < 1e-9
+
+
+@pytest.mark.parametrize("fmt", [0, 1])
+def test_many_points_with_duplicates_bitwise_vs_oracle(cuda_device, fmt):
+    """210 receiver entries (more than a block of threads), cells named several
+    times within a shot and by several shots, injected as adjoint sources: added
+    in entry order, equal bits to the oracle; FP32 and BF16 snapshots."""
+    pb = _problem(57, 9, 10, 11, 3, 24, n_rec=70)
+    pb.receivers_i[:, 40] = pb.receivers_i[:, 3]
+    pb.receivers_i[:, 69] = pb.receivers_i[:, 3]
+    pb.receivers_i[1:] = torch.where(torch.arange(70) % 2 == 0, pb.receivers_i[:1],
+                                     pb.receivers_i[1:])
+    g, r, sn = _fwd_store(pb, cuda_device, fmt)
+    grad_r = torch.randn((pb.nt, pb.n_shots, pb.n_rec), generator=torch.Generator().manual_seed(4))
+    gca, gcb, gf = em3d.native_backward(g, g.ca, g.cb, grad_r.to(cuda_device), sn, True, True, True)
+    torch.cuda.synchronize()
+    sdt = torch.bfloat16 if fmt else torch.float32
+    st_o = [torch.zeros((pb.nt, pb.n_shots, pb.nz, pb.ny, pb.nx), dtype=sdt) for _ in range(6)]
+    r_o = torch.zeros((pb.nt, pb.n_shots, pb.n_rec))
+    f_o, m_o = Oracle3D.full_state(pb)
+    o = Oracle3D()
+    o.forward(pb, pb.ca, pb.cb, pb.f, r_o, f_o, m_o, store=st_o, k=1, fmt=fmt)
+    oca, ocb, ogf, *_ = o.backward(pb, pb.ca, pb.cb, grad_r, st_o, k=1, fmt=fmt)
+    _same(r, r_o, "receivers")
+    _same(gca.reshape(oca.shape), oca, "grad ca")
+    _same(gcb.reshape(ocb.shape), ocb, "grad cb")
+    _same(gf.reshape(ogf.shape), ogf, "grad f")
+    assert nat.device_status(cuda_device) == 0
