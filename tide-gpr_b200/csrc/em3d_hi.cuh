@@ -331,7 +331,7 @@ k3p_adj_e(G3<T> g, const T *__restrict__ cb, const T *__restrict__ lex,
     const T b = ld(cb + j);
     const T lx = ld(lex + j), ly = ld(ley + j), lz = ld(lez + j);
     const T qx = b * lx, qy = b * ly, qz = b * lz;
-    fold_grad(g, gf, base + j, j, lx, ly, lz);
+    fold_add(g, gf, fold_load(g, gf, base + j), base + j, lx, ly, lz);
     if (z < g.z0 || z >= g.z1) {
       const int64_t m = pmi<T, 0>(g, z, y, x);
       const T bz = ld(g.p[PBZ] + z);
