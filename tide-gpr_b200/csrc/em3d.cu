@@ -147,14 +147,20 @@ __device__ __forceinline__ Prof<T> prof_at(const G3<T> &g, int pa, int pk, int c
   return Prof<T>{ld(g.p[pa] + c), ld(g.p[pa + 1] + c), ld(g.p[pk] + c)};
 }
 
-// Operands of one forward-H cell, loaded one cell ahead of its arithmetic so
-// that two cells' loads are in flight per thread.
+// Operands of one forward-H cell.  Its CPML memories are loaded with them, before
+// any arithmetic: read where each derivative is corrected, they were waited for one
+// after another, up to six times a strip cell, and the strips are over half of a
+// grid of this size.  Half step of 2 x (115 x 136 x 150) / 4 x 153^3 FP32 cells: 85 /
+// 204 us before, 71 / 189 with the cell's loads together and none ahead, 74 / 195 with
+// the other operands also a cell ahead (two cells of them do not fit 64 registers).
+// 48 and 40 registers spill (85 / 222 and 93 / 243); 4, 8 or 16 cells a run and 2, 4
+// or 8 rows a block lie within 6 percent.
 template <typename T> struct OpsH {
   T q, e_z, n_x, n_y, ez_y, ex_y, ez_x, ey_x, h_x, h_y, h_z;
 };
 
 template <typename T>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(32 * kBlockY3, 8)
 k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *__restrict__ ey,
          const T *__restrict__ ez, T *__restrict__ hx, T *__restrict__ hy, T *__restrict__ hz,
          T *__restrict__ m_ey_z, T *__restrict__ m_ez_y, T *__restrict__ m_ez_x,
@@ -170,8 +176,8 @@ k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *_
   m_ez_y += c.s * msz1(g); m_ex_y += c.s * msz1(g);
   m_ez_x += c.s * msz2(g); m_ey_x += c.s * msz2(g);
   const bool yok = y < ny - 1, xok = x < nx - 1;
-  const bool py = y < g.y0 || y >= g.y1h, px = x < g.x0 || x >= g.x1h;
-  const Prof<T> fy = prof_at(g, PAYH, PKYH, y, py && yok), fx = prof_at(g, PAXH, PKXH, x, px && xok);
+  const bool py = yok && (y < g.y0 || y >= g.y1h), px = xok && (x < g.x0 || x >= g.x1h);
+  const Prof<T> fy = prof_at(g, PAYH, PKYH, y, py), fx = prof_at(g, PAXH, PKXH, x, px);
   const int64_t o1 = (int64_t)ccoord(y, g.y0, g.yhs) * nx + x, s1 = (int64_t)g.eyc * nx;
   const int64_t o2 = (int64_t)y * g.exc + ccoord(x, g.x0, g.xhs), s2 = (int64_t)ny * g.exc;
   auto load = [&](int z, int64_t jj) {
@@ -197,23 +203,37 @@ k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *_
   };
   int64_t j = ((int64_t)c.zb * ny + y) * nx + x;
   T e_x = ld(ex + j), e_y = ld(ey + j);
-  OpsH<T> o = load(c.zb, j);
   for (int z = c.zb; z < c.ze; ++z, j += sz) {
-    OpsH<T> on{};
-    if (z + 1 < c.ze) on = load(z + 1, j + sz);
+    const OpsH<T> o = load(z, j);
+    // the cell's CPML memories before its arithmetic: their loads are in flight together
+    const bool pz = z < nz - 1 && (z < g.z0 || z >= g.z1h);
+    const int64_t mz = ((int64_t)ccoord(z, g.z0, g.zhs) * ny + y) * nx + x;
+    const int64_t my = z * s1 + o1, mx = z * s2 + o2;
+    T v_eyz = 0, v_exz = 0, v_ezy = 0, v_exy = 0, v_ezx = 0, v_eyx = 0;
+    if (pz) {
+      v_eyz = m_ey_z[mz];
+      v_exz = m_ex_z[mz];
+    }
+    if (py) {
+      v_ezy = m_ez_y[my];
+      v_exy = m_ex_y[my];
+    }
+    if (px) {
+      v_ezx = m_ez_x[mx];
+      v_eyx = m_ey_x[mx];
+    }
     T dEy_dz = 0, dEz_dy = 0, dEz_dx = 0, dEx_dz = 0, dEx_dy = 0, dEy_dx = 0;
     if (z < nz - 1) {
       T d = (o.n_y - e_y) * g.rdz;
       T d2 = (o.n_x - e_x) * g.rdz;
-      if (z < g.z0 || z >= g.z1h) {
-        const int64_t m = ((int64_t)ccoord(z, g.z0, g.zhs) * ny + y) * nx + x;
-        const T b = ld(g.p[PBZH] + z), a = ld(g.p[PAZH] + z), k = ld(g.p[PKZH] + z);
-        const T m1 = b * m_ey_z[m] + a * d;
-        m_ey_z[m] = m1;
-        d = div_k(d, k) + m1;
-        const T m2 = b * m_ex_z[m] + a * d2;
-        m_ex_z[m] = m2;
-        d2 = div_k(d2, k) + m2;
+      if (pz) {
+        const Prof<T> fz = prof_at(g, PAZH, PKZH, z, true);
+        const T m1 = fz.b * v_eyz + fz.a * d;
+        m_ey_z[mz] = m1;
+        d = div_k(d, fz.k) + m1;
+        const T m2 = fz.b * v_exz + fz.a * d2;
+        m_ex_z[mz] = m2;
+        d2 = div_k(d2, fz.k) + m2;
       }
       dEy_dz = d;
       dEx_dz = d2;
@@ -222,12 +242,11 @@ k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *_
       T d = (o.ez_y - o.e_z) * g.rdy;
       T d2 = (o.ex_y - e_x) * g.rdy;
       if (py) {
-        const int64_t m = z * s1 + o1;
-        const T m1 = fy.b * m_ez_y[m] + fy.a * d;
-        m_ez_y[m] = m1;
+        const T m1 = fy.b * v_ezy + fy.a * d;
+        m_ez_y[my] = m1;
         d = div_k(d, fy.k) + m1;
-        const T m2 = fy.b * m_ex_y[m] + fy.a * d2;
-        m_ex_y[m] = m2;
+        const T m2 = fy.b * v_exy + fy.a * d2;
+        m_ex_y[my] = m2;
         d2 = div_k(d2, fy.k) + m2;
       }
       dEz_dy = d;
@@ -237,12 +256,11 @@ k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *_
       T d = (o.ez_x - o.e_z) * g.rdx;
       T d2 = (o.ey_x - e_y) * g.rdx;
       if (px) {
-        const int64_t m = z * s2 + o2;
-        const T m1 = fx.b * m_ez_x[m] + fx.a * d;
-        m_ez_x[m] = m1;
+        const T m1 = fx.b * v_ezx + fx.a * d;
+        m_ez_x[mx] = m1;
         d = div_k(d, fx.k) + m1;
-        const T m2 = fx.b * m_ey_x[m] + fx.a * d2;
-        m_ey_x[m] = m2;
+        const T m2 = fx.b * v_eyx + fx.a * d2;
+        m_ey_x[mx] = m2;
         d2 = div_k(d2, fx.k) + m2;
       }
       dEz_dx = d;
@@ -253,17 +271,20 @@ k3_fwd_h(G3<T> g, const T *__restrict__ cq, const T *__restrict__ ex, const T *_
     hz[j] = o.h_z - o.q * (dEx_dy - dEy_dx);
     e_x = o.n_x;
     e_y = o.n_y;
-    o = on;
   }
 }
 
-// Operands of one forward-E cell (loaded one cell ahead, as OpsH).
+// Operands of one forward-E cell, loaded one cell ahead of the arithmetic; the
+// CPML memories of the cell itself are loaded together before it, as in the H sweep.
+// Half step of 2 x (115 x 136 x 150) / 4 x 153^3 FP32 cells: 87 / 211 us with each
+// memory read at its derivative, 73 / 190 now (252 -> 229 storing BF16 snapshots);
+// 75 / 199 (237) without the operands a cell ahead.
 template <typename T> struct OpsE {
   T a, b, h_x, h_y, h_z, hz_y, hz_x, hx_y, hy_x, e_x, e_y, e_z;
 };
 
 template <typename T, typename S>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(32 * kBlockY3, 8)
 k3_fwd_e(G3<T> g, const T *__restrict__ ca, const T *__restrict__ cb, T *__restrict__ ex,
          T *__restrict__ ey, T *__restrict__ ez, const T *__restrict__ hx,
          const T *__restrict__ hy, const T *__restrict__ hz, T *__restrict__ m_hz_y,
@@ -311,38 +332,52 @@ k3_fwd_e(G3<T> g, const T *__restrict__ ca, const T *__restrict__ cb, T *__restr
   for (int z = c.zb; z < c.ze; ++z, j += sz) {
     OpsE<T> on{};
     if (z + 1 < c.ze) on = load(j + sz);
+    // the cell's CPML memories before its arithmetic, as in k3_fwd_h
+    const bool pz = z < g.z0 || z >= g.z1;
+    const int64_t mz = ((int64_t)ccoord(z, g.z0, g.zhs) * ny + y) * nx + x;
+    const int64_t my = z * s1 + o1, mx = z * s2 + o2;
+    T v_hyz = 0, v_hxz = 0, v_hzy = 0, v_hxy = 0, v_hzx = 0, v_hyx = 0;
+    if (pz) {
+      v_hyz = m_hy_z[mz];
+      v_hxz = m_hx_z[mz];
+    }
+    if (py) {
+      v_hzy = m_hz_y[my];
+      v_hxy = m_hx_y[my];
+    }
+    if (px) {
+      v_hzx = m_hz_x[mx];
+      v_hyx = m_hy_x[mx];
+    }
     T dHy_dz = (o.h_y - p_y) * g.rdz;
     T dHz_dy = (o.h_z - o.hz_y) * g.rdy;
     T dHz_dx = (o.h_z - o.hz_x) * g.rdx;
     T dHx_dz = (o.h_x - p_x) * g.rdz;
     T dHx_dy = (o.h_x - o.hx_y) * g.rdy;
     T dHy_dx = (o.h_y - o.hy_x) * g.rdx;
-    if (z < g.z0 || z >= g.z1) {
-      const int64_t m = ((int64_t)ccoord(z, g.z0, g.zhs) * ny + y) * nx + x;
-      const T bb = ld(g.p[PBZ] + z), aa = ld(g.p[PAZ] + z), k = ld(g.p[PKZ] + z);
-      const T m1 = bb * m_hy_z[m] + aa * dHy_dz;
-      m_hy_z[m] = m1;
-      dHy_dz = div_k(dHy_dz, k) + m1;
-      const T m2 = bb * m_hx_z[m] + aa * dHx_dz;
-      m_hx_z[m] = m2;
-      dHx_dz = div_k(dHx_dz, k) + m2;
+    if (pz) {
+      const Prof<T> fz = prof_at(g, PAZ, PKZ, z, true);
+      const T m1 = fz.b * v_hyz + fz.a * dHy_dz;
+      m_hy_z[mz] = m1;
+      dHy_dz = div_k(dHy_dz, fz.k) + m1;
+      const T m2 = fz.b * v_hxz + fz.a * dHx_dz;
+      m_hx_z[mz] = m2;
+      dHx_dz = div_k(dHx_dz, fz.k) + m2;
     }
     if (py) {
-      const int64_t m = z * s1 + o1;
-      const T m1 = fy.b * m_hz_y[m] + fy.a * dHz_dy;
-      m_hz_y[m] = m1;
+      const T m1 = fy.b * v_hzy + fy.a * dHz_dy;
+      m_hz_y[my] = m1;
       dHz_dy = div_k(dHz_dy, fy.k) + m1;
-      const T m2 = fy.b * m_hx_y[m] + fy.a * dHx_dy;
-      m_hx_y[m] = m2;
+      const T m2 = fy.b * v_hxy + fy.a * dHx_dy;
+      m_hx_y[my] = m2;
       dHx_dy = div_k(dHx_dy, fy.k) + m2;
     }
     if (px) {
-      const int64_t m = z * s2 + o2;
-      const T m1 = fx.b * m_hz_x[m] + fx.a * dHz_dx;
-      m_hz_x[m] = m1;
+      const T m1 = fx.b * v_hzx + fx.a * dHz_dx;
+      m_hz_x[mx] = m1;
       dHz_dx = div_k(dHz_dx, fx.k) + m1;
-      const T m2 = fx.b * m_hy_x[m] + fx.a * dHy_dx;
-      m_hy_x[m] = m2;
+      const T m2 = fx.b * v_hyx + fx.a * dHy_dx;
+      m_hy_x[mx] = m2;
       dHy_dx = div_k(dHy_dx, fx.k) + m2;
     }
     const T cx = dHy_dz - dHz_dy, cy = dHz_dx - dHx_dz, cz = dHx_dy - dHy_dx;
@@ -777,7 +812,7 @@ template <typename T> struct OpsAH {
 // outside the update domain and on the last plane of their axis); the own
 // z terms of a cell are the z - 1 terms of the next cell of the march.
 template <typename T>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(32 * kBlockY3, 6)
 k3_adj_h(G3<T> g, const T *__restrict__ ca, const T *__restrict__ cq,
          const T *__restrict__ lhx, const T *__restrict__ lhy, const T *__restrict__ lhz,
          T *__restrict__ lex, T *__restrict__ ley, T *__restrict__ lez, Mem12<T> cur,
