@@ -141,6 +141,15 @@ struct Scratch {
   }
 };
 
+// True where the device has no memory for the scratch: nothing was launched, and the
+// per-step kernels, which need less, take the call.
+bool scratch_alloc(Scratch &sc, size_t bytes) {
+  if (pool_malloc(&sc.p, bytes, sc.st) == cudaSuccess) return false;
+  cudaGetLastError();
+  sc.p = nullptr;
+  return true;
+}
+
 template <typename Args>
 ResRun launch(void (*k)(const Args), const Args &a, cudaStream_t st) {
   if (TB_CUDA(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -168,7 +177,7 @@ ResRun run_forward(const ResFwdCall &c, const ResPlan &pl) {
   if (lists > ((size_t)256 << 20)) return ResRun::kNotTaken;
   Scratch sc;
   sc.st = c.st;
-  if (TB_CUDA(pool_malloc(&sc.p, ll + lists + 16, c.st))) return ResRun::kFailed;
+  if (scratch_alloc(sc, ll + lists + 16)) return ResRun::kNotTaken;
   if (ll && TB_CUDA(cudaMemsetAsync(sc.p, 0, ll, c.st))) return ResRun::kFailed;
   ResFwdArgs<Sn> a{};
   a.g = g;
@@ -208,7 +217,7 @@ ResRun run_backward(const ResAdjCall &c, const ResPlan &pl) {
   if (lists > ((size_t)256 << 20)) return ResRun::kNotTaken;
   Scratch sc;
   sc.st = c.st;
-  if (TB_CUDA(pool_malloc(&sc.p, ll + n_acc * acc + lists + 16, c.st))) return ResRun::kFailed;
+  if (scratch_alloc(sc, ll + n_acc * acc + lists + 16)) return ResRun::kNotTaken;
   if (ll && TB_CUDA(cudaMemsetAsync(sc.p, 0, ll, c.st))) return ResRun::kFailed;
   char *m = static_cast<char *>(sc.p) + ll;
   ResAdjArgs<Sn> a{};
